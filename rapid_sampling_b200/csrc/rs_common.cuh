@@ -262,6 +262,41 @@ __device__ __forceinline__ float4 scaled4_rep(float4 l, float4 q, float scale) {
                         scaled_logit(l.z, q.z, true, scale), scaled_logit(l.w, q.w, true, scale));
     return v;
 }
+// Correctly rounded quotients by one denominator (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990): y is the correctly rounded 1/b; the first correction makes q a
+// neighbour of a/b (what it rounds is within 1.5 ulp * 2^-24 of a/b), and for such a q with an exact remainder the second
+// one yields the rounded quotient.  Remainders are exact and nothing underflows for a >= kDivMin (a multiple of a's last
+// place times 2^-24 stays normal); a = 0 gives 0.  Five fused operations instead of a call of the general division
+// with its reciprocal and its range test per element; the same bits (tests/test_division.py repeats the steps exactly).
+constexpr float kDivMin = 1.0e-24f;
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+    float q = a * y;
+    q = fmaf(fmaf(-q, b, a), y, q);
+    return fmaf(fmaf(-q, b, a), y, q);
+}
+// Four probabilities exp2f(x - mx) / denom of a group (y = the rounded 1 / denom).
+__device__ __forceinline__ float4 prob4(float4 v, float mx, float denom, float y) {
+    v.x = exp2f(v.x - mx); v.y = exp2f(v.y - mx); v.z = exp2f(v.z - mx); v.w = exp2f(v.w - mx);
+    if (fminf(fminf(v.x, v.y), fminf(v.z, v.w)) >= kDivMin)
+        return make_float4(div_by(v.x, denom, y), div_by(v.y, denom, y), div_by(v.z, denom, y), div_by(v.w, denom, y));
+    return make_float4(v.x / denom, v.y / denom, v.z / denom, v.w / denom);
+}
+
+// Adds one group of a row of which nothing is cut off to a lane's ordered mass above the threshold (the smallest
+// probability of the row) and counts its ties.
+__device__ __forceinline__ void add_open(float4 v, float thr, float& gtp, uint32_t& eqk) {
+    const float e[4] = {v.x, v.y, v.z, v.w};
+    if (fminf(fminf(v.x, v.y), fminf(v.z, v.w)) > thr) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) gtp += e[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (e[i] > thr) gtp += e[i];
+            else eqk++;
+        }
+    }
+}
 // Appends the candidates of one float4 group to the lane's list (rare; out of line).
 __device__ __forceinline__ void append_candidates(float4 v, float beta_e, float* list, int stride4, int cap, int& nc, int& ns) {
     const float e[4] = {v.x, v.y, v.z, v.w};

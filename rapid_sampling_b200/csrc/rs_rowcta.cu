@@ -757,6 +757,9 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
     uint32_t eqk[LPT], gtk[LPT];
 #pragma unroll
     for (int j = 0; j < LPT; j++) { gtp[j] = 0.f; eqk[j] = 0u; gtk[j] = 0u; }
+    // no test of the search loop can hold from the start: no top_k below V and no top_p below 1
+    const bool open_row = top_p >= 1.0f && (!use_cnt || top_k >= (uint32_t)V);
+    const float emin_up = fmaxf(emin * 1.000001f, kDivMin);   // a numerator above it has a quotient above pmin (8 ulp apart)
     // Two attempts share one copy of the search loop: the candidate lists first (the first CR probabilities of every
     // lane's list live in registers for the rounds -- unused places hold -1, which no pivot admits -- longer lists
     // continue in shared memory), then, if they cannot settle the cutoff, the whole row on the global scratch row.
@@ -883,6 +886,47 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
                     const int vl = j * NT + t;
                     eqk[j] = (vl < V4) ? (uint32_t)(((V4 - vl + kLanes - 1) >> 10) * 4) : 0u;
                 }
+                break;
+            }
+            if (open_row) {
+                // Nothing is cut off: the reference's loop never starts (sampling.cu:598) and leaves left = pmin.  What is
+                // left of its work is the recount, so the probabilities are summed as they are computed and never stored.
+                // The threshold is the smallest of them: all others lie above it.
+                left = __float_as_uint(pmin);
+                right = __float_as_uint(pmax) + 1u;
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                begin_pass(NC, 1, Yes(), Pen());
+                const float inv = __frcp_rn(denom);
+                stream_x([&](const int j, const int, const float4 v) { add_open(prob4(v, mx, denom, inv), pmin, gtp[j], eqk[j]); },
+                         [&](const int h, const int, float4 (&v)[SL]) {
+                             float lo = INFINITY;
+#pragma unroll
+                             for (int jj = 0; jj < SL; jj++) {
+                                 v[jj].x = exp2f(v[jj].x - mx); v[jj].y = exp2f(v[jj].y - mx);
+                                 v[jj].z = exp2f(v[jj].z - mx); v[jj].w = exp2f(v[jj].w - mx);
+                                 lo = fminf(fminf(lo, fminf(v[jj].x, v[jj].y)), fminf(v[jj].z, v[jj].w));
+                             }
+                             if (lo > emin_up) {   // every quotient of the stage lies above pmin
+#pragma unroll
+                                 for (int jj = 0; jj < SL; jj++) {
+                                     float& g = gtp[h * SL + jj];
+                                     g += div_by(v[jj].x, denom, inv); g += div_by(v[jj].y, denom, inv);
+                                     g += div_by(v[jj].z, denom, inv); g += div_by(v[jj].w, denom, inv);
+                                 }
+                             } else {
+#pragma unroll
+                                 for (int jj = 0; jj < SL; jj++)
+                                     add_open(make_float4(v[jj].x / denom, v[jj].y / denom, v[jj].z / denom, v[jj].w / denom), pmin,
+                                              gtp[h * SL + jj], eqk[h * SL + jj]);
+                             }
+                         });
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < LPT; j++) {
+                    const int vl = j * NT + t;
+                    gtk[j] = ((vl < V4) ? (uint32_t)(((V4 - vl + kLanes - 1) >> 10) * 4) : 0u) - eqk[j];
+                }
+                if (REP) begin_pass(K - 1, -1, No(), Yes());
                 break;
             }
             // p = exp2f(x - max) / denom (sampling.cu:573-590) into the global scratch row

@@ -751,6 +751,16 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         left = __float_as_uint(pmin);
         right = left + 1u;
         eqk = (uint32_t)(Kt * 4);
+    } else if (!done && top_p >= 1.0f && (!use_cnt || top_k >= (uint32_t)V)) {
+        // Nothing is cut off: the reference's loop never starts (sampling.cu:598) and leaves left = pmin.  What is left
+        // of its work is the recount, so the probabilities are summed as they are computed and never stored (B=256,
+        // V=151936: 155.7 -> 100.9 us; the scratch row cost a write and a read of 155 MB and the general division).
+        left = __float_as_uint(pmin);
+        right = __float_as_uint(pmax) + 1u;
+        const float inv = __frcp_rn(denom);
+#pragma unroll 4
+        for (int s = 0; s < Kt; s++) add_open(prob4(xload(s), mx, denom, inv), pmin, gtp, eqk);
+        gtk = (uint32_t)(Kt * 4) - eqk;
     } else if (!done) {
         // ===== whole row: pass 3, p = exp2f(x - max) / denom (sampling.cu:573-590), in place; then the search
         // over every lane's full list, dropping elements below `left` as the bracket rises =====

@@ -1,0 +1,55 @@
+"""Search paths of the sampler kernels at the sizes where they can go wrong: the CPU oracle, fed the kernel's own fp32
+probabilities and RNG states, must land on the same bits (threshold, totals, weights, id)."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import make_logits
+from oracle import c_oracle as co
+
+pytestmark = pytest.mark.gpu
+
+FIELDS_U = ("left", "seqk", "sgtk", "rounds", "idxt", "early_exit")
+FIELDS_F = ("threshold", "comp", "sgtp", "sum_p", "randp", "sum_o", "rand2", "pmin", "pmax")
+
+
+def check_against_oracle(abi, lg, seed, temp, k, p, mode=0, pen=None, rows=4):
+    B, V = lg.shape
+    st = abi.setup_rand(seed, B)
+    st_cpu = st.cpu().numpy().copy()
+    pen_dev = pen.clone().cuda() if pen is not None else None
+    abi.set_path(mode)
+    try:
+        out, probs, tr = abi.sample(lg.cuda(), st, temp, k, p, penalties=pen_dev, presence=0.1, repetition=0.1, decay=0.95, debug=True)
+    finally:
+        abi.set_path(0)
+    knd, scale, kk, pp = co.normalise(V, B, 1, temp, k, p, with_penalties=pen is not None)
+    for b in sorted({0, B - 1, B // 2, B // 3})[:rows]:
+        pen_cpu = pen[b].numpy().copy() if pen is not None else None
+        tok, o, _ = co.sample_row(lg[b].numpy(), st_cpu[64 * b:64 * b + 64], knd, scale, kk, pp, penalties=pen_cpu, presence=0.1,
+                                  repetition=0.1, decay=0.95, probs_in=probs[b].cpu().numpy())
+        g = tr[b]
+        assert tok == int(out[b]) == g.token, b
+        for f in FIELDS_U:
+            assert getattr(o, f) == getattr(g, f), (b, f, getattr(o, f), getattr(g, f))
+        for f in FIELDS_F:
+            x, y = np.float32(getattr(o, f)), np.float32(getattr(g, f))
+            assert x.view(np.uint32) == y.view(np.uint32), (b, f, x, y)
+        if pen is not None:
+            assert np.array_equal(pen_cpu, pen_dev[b].cpu().numpy())
+    assert abi.device_status() == 0
+    return tr
+
+
+@pytest.mark.parametrize("mode", [0, 2, 3, 4])        # the planner's choice, streaming, on-chip, one CTA per row
+@pytest.mark.parametrize("kind,B,V,temp", [("normal3", 3, 4, 1.0), ("peaked", 130, 4096, 1.0), ("uniform", 4, 4100, 0.7),
+                                           ("coarse", 300, 8188, 1.0), ("special", 5, 50304, 1.3), ("equal", 4, 8192, 1.0),
+                                           ("normal3", 2, 65536, 0.02)])
+def test_rows_of_which_nothing_is_cut_off(abi, mode, kind, B, V, temp):
+    """No top_k and top_p = 1: the recount runs on probabilities that are never stored (and, at temperature 0.02, on
+    numerators too small for the short division)."""
+    tr = check_against_oracle(abi, make_logits(kind, B, V, 11, torch), 5, temp, -1, 1.0, mode)
+    assert all(t.rounds == 0 for t in tr)
+    if mode in (0, 4):
+        pen = torch.rand(B, V, generator=torch.Generator().manual_seed(1)) * 0.5
+        check_against_oracle(abi, make_logits(kind, B, V, 12, torch), 6, temp, -1, 1.0, mode, pen=pen)
