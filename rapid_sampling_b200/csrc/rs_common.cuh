@@ -45,8 +45,9 @@ constexpr int kXStride = 12;                     // words between two warps' rec
 constexpr int kMboxOff = 0;                      // 2 buffers of [32 warps][kXStride] words
 constexpr int kMboxBuf = kXStride * 32 * 4;
 constexpr int kMiscOff = 2 * kMboxBuf;           // mbarriers, small scalars, 32 warp totals
-constexpr int kQuickCap = 512;                   // longest candidate list the one-warp search takes
-constexpr int kQuickOff = kMiscOff + 256;        // the row's candidates as one unordered list of (bits of p, p in units of 2^-30)
+constexpr int kQuickCap = 512;                   // longest candidate list the search on integer masses takes
+constexpr int kQsumOff = kMiscOff + 256;         // counts and masses at that search's 32 samples
+constexpr int kQuickOff = kQsumOff + 256;        // the row's candidates as one unordered list of (bits of p, p in units of 2^-30)
 constexpr int kSlabOff = kQuickOff + kQuickCap * 8;
 constexpr uint32_t kDefaultWaitPolls = 1u << 22;
 
@@ -115,120 +116,140 @@ __device__ __forceinline__ void slab_pass(const Row<C, SMEM>& row, int& n, const
     c23 = cw;
 }
 
-// ---- the cutoff search of a whole row's candidate list in ONE warp, on integer masses ---------------------------
+// ---- the cutoff search of a whole row's candidate list, on integer masses ---------------------------------------
 // The reference's loop only ever asks whether a mass is below or above top_p (sampling.cu:598, :618-651).  `list`
 // holds every candidate of the row as (bits of p, p in units of 2^-30), in any order: the sum of the admitted
 // entries' second words is exact up to half a unit per entry and does not depend on the order.  The reference's fp32
 // value differs from the true sum by at most one rounding per addition on the longest path (`depth`: the entries of
-// one lane, 5 in the warp tree, 31 over the warps).  Outside that margin around top_p the answer is certain and the
-// loop is replayed here -- same pivots, same tests, same bracket updates -- without any exchange; inside it (unless a
-// count decides the test anyway) the verdict is 0 and the caller runs the exact search from the start.
+// one lane, 5 in the warp tree, 31 over the warps).  Outside that margin around top_p the answer is certain; inside it
+// (unless a count decides the test anyway) the verdict is 0 and the caller runs the exact search from the start.
 // Pivots at or below beta_p are answered by the set {p > beta_p}, as in the exact search on a candidate list.
-// All 32 lanes call this with the same arguments; `list` must be readable up to the next multiple of 256 entries
-// (entries from n on are overwritten with "never admitted").
-// FREEZE: once the sets at `left` and at `right` differ by at most one entry, the remaining rounds are replayed from the
-// carried values without reading the list (pays where rounds are many; costs registers).
+//
+// The answer at a pivot u depends only on the set {p >= u}, which shrinks as u rises: every entry up to some x2 has a
+// set that exceeds top_k or top_p, every entry above some x has one that passes, and between the two lie those where
+// neither is certain.  So x2 and x are found first and the loop is then replayed -- same pivots, same tests, same
+// bracket updates -- on two integer compares per test, without reading the list.  x2 and x are found by rank: 32
+// entries of the list as sample, each lane sums the sets of one of them (quick_sample: the list is split over the warps
+// of the CTA), which leaves about a thirty-second of the list between the highest sample that exceeds and the lowest
+// that passes; one warp ranks those against each other (quick_settle).  Bound by the latency of one warp: replaying the
+// loop with a scan of the list in each of its ~14 rounds took 2 us longer (a call of B=1, V=262144: 20.0 -> 18.2 us;
+// B=160, V=100256, bf16: 51.0 -> 46.7 us).
+struct QuickTest {       // the three possible outcomes of the reference's tests at a set of count c and mass m
+    bool use_cnt;
+    uint32_t top_k, tp_lo, tp_hi, margin;
+    __device__ __forceinline__ QuickTest(bool uc, uint32_t k, float top_p, int depth) {
+        use_cnt = uc;
+        top_k = k;
+        margin = (uint32_t)(depth * 66 + kQuickCap / 2 + 8);
+        tp_lo = __float2uint_rd(top_p * 1073741824.f);
+        tp_hi = __float2uint_ru(top_p * 1073741824.f);
+    }
+    // 2: more than top_k entries or more than top_p mass for certain; 0: fewer and less for certain; 1: neither test
+    // (count equal to top_k); 3: the mass is too close to top_p to tell
+    __device__ __forceinline__ int operator()(uint32_t c, uint32_t m) const {
+        const bool lt = m + margin < tp_lo, gt = m > tp_hi + margin, many = use_cnt && c > top_k;
+        if (gt || many) return 2;
+        if (!lt) return 3;
+        return (!use_cnt || c < top_k) ? 0 : 1;
+    }
+};
+
+// First part, all NW warps of the CTA: counts and masses at the 32 samples into sums[0..31], sums[32..63] (cleared by
+// the caller; complete after the next CTA barrier).
+template <int NW>
+__device__ __forceinline__ void quick_sample(const uint2* list, const uint32_t n, const int w, const int lane, uint32_t* sums) {
+    const uint32_t pv = list[((uint32_t)lane * n) >> 5].x;
+    const uint32_t chunk = (n + NW - 1) / NW, i0 = (uint32_t)w * chunk, i1 = min(n, i0 + chunk);
+    uint32_t c = 0u, m = 0u;
+#pragma unroll 8
+    for (uint32_t i = i0; i < i1; i++) {
+        const uint2 e = list[i];
+        if (e.x >= pv) { c++; m += e.y; }
+    }
+    atomicAdd(sums + lane, c);
+    atomicAdd(sums + 32 + lane, m);
+}
+
+// Second part, one warp (all 32 lanes, same arguments).  The list is compacted in place.
 // Verdict: 1 settled (left / right / rounds are the reference's), 2 the list cannot settle the cutoff, 0 undecided.
-template <bool FREEZE>
-__device__ __forceinline__ int quick_search(uint2* list, const uint32_t n, const int lane, const int depth, const bool use_cnt,
-                                            const uint32_t top_k, const float top_p, const uint32_t beta_p, const float pmin,
-                                            const float pmax, const uint32_t V, uint32_t& left, uint32_t& right, uint32_t& rounds) {
+__device__ __forceinline__ int quick_settle(uint2* list, const uint32_t n, const int lane, const uint32_t* sums, const QuickTest test,
+                                            const float top_p, const uint32_t beta_p, const float pmin, const float pmax,
+                                            const uint32_t V, uint32_t& left, uint32_t& right, uint32_t& rounds) {
     constexpr unsigned FULLW = 0xffffffffu;
-    for (uint32_t i = n + (uint32_t)lane; i < ((n + 255u) & ~255u); i += 32u) list[i] = make_uint2(0u, 0u);
-    __syncwarp();
-    const uint32_t margin = (uint32_t)(depth * 66 + kQuickCap / 2 + 8);
-    const uint32_t tp_lo = __float2uint_rd(top_p * 1073741824.f), tp_hi = __float2uint_ru(top_p * 1073741824.f);
+    uint32_t x2 = 0u;                                    // every entry up to here exceeds
+    uint32_t x0 = 0xffffffffu, base_c = 0u, base_m = 0u; // every entry from here on passes; count and mass of that set
+    uint32_t nz = n, pv = list[((uint32_t)lane * n) >> 5].x, c = sums[lane], m = sums[32 + lane];
+    for (int it = 0;; it++) {
+        const int cls = test(c, m);
+        x2 = max(x2, __reduce_max_sync(FULLW, cls == 2 ? pv : 0u));
+        const uint32_t low = __reduce_min_sync(FULLW, cls == 0 ? pv : 0xffffffffu);
+        if (low < x0) {
+            const int src = __ffs(__ballot_sync(FULLW, cls == 0 && pv == low)) - 1;
+            x0 = low;
+            base_c = __shfl_sync(FULLW, c, src);
+            base_m = __shfl_sync(FULLW, m, src);
+        }
+        // what lies between: compacted to the front of the list (a place is written only after it has been read)
+        const uint32_t lo = max(x2, beta_p);
+        uint32_t q = 0u;
+        for (uint32_t i0 = 0u; i0 < nz; i0 += 32u) {
+            const uint32_t i = i0 + (uint32_t)lane;
+            const uint2 e = (i < nz) ? list[i] : make_uint2(0u, 0u);
+            const bool in = e.x > lo && e.x < x0;
+            const unsigned b = __ballot_sync(FULLW, in);
+            __syncwarp();
+            if (in) list[q + (uint32_t)__popc(b & ((1u << lane) - 1u))] = e;
+            q += (uint32_t)__popc(b);
+        }
+        __syncwarp();
+        nz = q;
+        if (nz <= 32u || it == 3) break;
+        pv = list[((uint32_t)lane * nz) >> 5].x;
+        c = base_c;
+        m = base_m;
+#pragma unroll 8
+        for (uint32_t i = 0u; i < nz; i++) {
+            const uint2 e = list[i];
+            if (e.x >= pv) { c++; m += e.y; }
+        }
+    }
+    uint32_t x = x2;
+    bool unsure = false;
+    for (uint32_t i0 = 0u; i0 < nz; i0 += 32u) {         // one turn (more only for masses of ties that cannot be told apart)
+        const bool mine = i0 + (uint32_t)lane < nz;
+        pv = mine ? list[i0 + (uint32_t)lane].x : 0xffffffffu;
+        c = base_c;
+        m = base_m;
+#pragma unroll 4
+        for (uint32_t i = 0u; i < nz; i++) {
+            const uint2 e = list[i];
+            if (e.x >= pv) { c++; m += e.y; }
+        }
+        const int cls = mine ? test(c, m) : 0;
+        x2 = max(x2, __reduce_max_sync(FULLW, cls == 2 ? pv : 0u));
+        x = max(x, __reduce_max_sync(FULLW, cls != 0 ? pv : 0u));
+        unsure = unsure || __any_sync(FULLW, cls == 3);
+    }
+    x = max(x, x2);
+    if (test(0u, 0u) != 0) { x = 0xffffffffu; unsure = true; }      // not even the empty set is clear of top_p
+
     const uint32_t ustar = beta_p + 1u;
     uint32_t l_left = __float_as_uint(pmin), l_right = __float_as_uint(pmax) + 1u, l_rounds = 0u;
-    // what the loop carries: the count at `left` and whether its mass is above top_p (the reference starts from the
-    // whole row and mass 1); kept beside it for the replay below: the same for `right` (nothing lies above pmax)
-    uint32_t cnt_x = V, cnt_r = 0u;
-    bool gt_x = 1.0f > top_p, lt_x = 1.0f < top_p, gt_r = false, lt_r = 0.0f < top_p;
-    bool have_x = false;                 // cnt_x counts list entries (left came from an evaluated pivot)
-    bool frozen = false;                 // at most one entry is left in [max(left, u*), right): no more scans
-    uint32_t v_bits = 0u;                // that entry (0: none; every evaluation point is above 0)
+    // whether the set at `left` keeps the loop going (the reference starts from the whole row and mass 1)
+    bool go = (test.use_cnt && V > test.top_k) || 1.0f > top_p;
     int verdict = 1;
-    for (;;) {
-        const bool go = use_cnt ? (cnt_x > top_k || gt_x) : gt_x;
-        if (!(go && l_left < l_right - 1u) || l_rounds >= 64u) break;
+    while (go && l_left < l_right - 1u && l_rounds < 64u) {
         l_rounds++;
         const uint32_t pz = (l_left + l_right) >> 1, py = (l_left + pz) >> 1, pwv = (pz + l_right) >> 1;
-        const uint32_t pv[3] = {py, pz, pwv};
-        const uint32_t ev[3] = {max(py, ustar), max(pz, ustar), max(pwv, ustar)};
-        uint32_t cnt[3];
-        bool lt[3], gt[3], unsure = false;
-        if (FREEZE && !frozen && have_x && cnt_x - cnt_r <= 1u) {
-            // The sets at `left` and at `right` differ by at most one entry, v: an evaluation point at or below v sees
-            // the set of `left`, one above v the set of `right`; the remaining rounds need no data.
-            frozen = true;
-            if (cnt_x != cnt_r) {
-                uint32_t m = 0u;
-                for (uint32_t i0 = 0u; i0 < n; i0 += 256u) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const uint32_t e = list[i0 + (uint32_t)(i * 32 + lane)].x;
-                        m = (e < l_right) ? max(m, e) : m;
-                    }
-                }
-                v_bits = __reduce_max_sync(FULLW, m);
-            }
-        }
-        if (FREEZE && frozen) {
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                const bool at_x = ev[i] <= v_bits;
-                cnt[i] = at_x ? cnt_x : cnt_r;
-                lt[i] = at_x ? lt_x : lt_r;
-                gt[i] = at_x ? gt_x : gt_r;
-            }
-        } else {
-            uint32_t c0 = 0u, c1 = 0u, c2 = 0u, q0 = 0u, q1 = 0u, q2 = 0u;
-            for (uint32_t i0 = 0u; i0 < n; i0 += 256u) {
-                uint2 en[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) en[i] = list[i0 + (uint32_t)(i * 32 + lane)];
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (en[i].x >= ev[0]) { c0++; q0 += en[i].y; }
-                    if (en[i].x >= ev[1]) { c1++; q1 += en[i].y; }
-                    if (en[i].x >= ev[2]) { c2++; q2 += en[i].y; }
-                }
-            }
-            cnt[0] = __reduce_add_sync(FULLW, c0); cnt[1] = __reduce_add_sync(FULLW, c1); cnt[2] = __reduce_add_sync(FULLW, c2);
-            const uint32_t qm[3] = {__reduce_add_sync(FULLW, q0), __reduce_add_sync(FULLW, q1), __reduce_add_sync(FULLW, q2)};
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                lt[i] = qm[i] + margin < tp_lo;
-                gt[i] = qm[i] > tp_hi + margin;
-                unsure = unsure || (!lt[i] && !gt[i] && !(use_cnt && cnt[i] > top_k));
-            }
-        }
-        if (unsure) { verdict = 0; break; }
-        bool ok[3], bad = false;
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const bool below = pv[i] <= beta_p;
-            const bool exceeds = (use_cnt && cnt[i] > top_k) || gt[i];
-            const bool pass = (!use_cnt || cnt[i] < top_k) && lt[i];
-            ok[i] = !below && pass;
-            bad = bad || (below && !exceeds);
-        }
-        if (bad) { verdict = 2; break; }
-        const bool s0 = ok[0], s1 = !s0 && ok[1], s2 = !s0 && !s1 && ok[2];
-        const uint32_t nl = s0 ? l_left : s1 ? pv[0] : s2 ? pv[1] : pv[2];
-        const uint32_t nr = s0 ? pv[0] : s1 ? pv[1] : s2 ? pv[2] : l_right;
-        const uint32_t ncx = s0 ? cnt_x : s1 ? cnt[0] : s2 ? cnt[1] : cnt[2];
-        const bool ngx = s0 ? gt_x : s1 ? gt[0] : s2 ? gt[1] : gt[2];
-        l_left = nl; l_right = nr;
-        cnt_x = ncx; gt_x = ngx;
-        if (FREEZE) {
-            const bool nlx = s0 ? lt_x : s1 ? lt[0] : s2 ? lt[1] : lt[2];
-            const uint32_t ncr = s0 ? cnt[0] : s1 ? cnt[1] : s2 ? cnt[2] : cnt_r;
-            const bool ngr = s0 ? gt[0] : s1 ? gt[1] : s2 ? gt[2] : gt_r;
-            const bool nlr = s0 ? lt[0] : s1 ? lt[1] : s2 ? lt[2] : lt_r;
-            have_x = have_x || !s0;
-            lt_x = nlx; cnt_r = ncr; gt_r = ngr; lt_r = nlr;
-        }
+        const uint32_t e0 = max(py, ustar), e1 = max(pz, ustar), e2 = max(pwv, ustar);
+        const bool g0 = e0 <= x2, g1 = e1 <= x2, g2 = e2 <= x2;     // exceeds
+        const bool s0 = e0 > x && py > beta_p, s1 = e1 > x && pz > beta_p, s2 = e2 > x && pwv > beta_p;   // passes
+        if (unsure && ((!g0 && e0 <= x) || (!g1 && e1 <= x) || (!g2 && e2 <= x))) { verdict = 0; break; }
+        if ((py <= beta_p && !g0) || (pz <= beta_p && !g1) || (pwv <= beta_p && !g2)) { verdict = 2; break; }
+        const uint32_t nl = s0 ? l_left : s1 ? py : s2 ? pz : pwv;
+        l_right = s0 ? py : s1 ? pz : s2 ? pwv : l_right;
+        l_left = nl;
+        go = s0 ? go : s1 ? g0 : s2 ? g1 : g2;
     }
     if (verdict == 1 && !(l_left > beta_p)) verdict = 2;
     left = l_left; right = l_right; rounds = l_rounds;

@@ -9,7 +9,7 @@
 //     16-byte copies (cp.async) into shared memory: several stripes in flight per thread, no registers held by loads
 //     in flight, and no barrier of any kind in the streaming passes.  The first stripes stay on chip as scaled logits,
 //     so the second pass re-reads only the rest (from L2);
-//   * the cutoff search runs on the short candidate list: first in one warp on exact integer masses, which settles
+//   * the cutoff search runs on the short candidate list: first on exact integer masses, which settles
 //     every row whose masses stay clear of top_p by more than the fp32 rounding of the reference's sums (nearly all);
 //     else with the reference's fp32 sums, block-wide, one CTA barrier per evaluated round;
 //   * with penalties, the first stripes of the update pass are already in flight while the search runs.
@@ -38,7 +38,8 @@ constexpr int kOffBoxC = 256;      // 2 x [16 physical warps][8 words]
 constexpr int kOffBox = 1280;      // 2 x [4 values][32 virtual warps] floats, value-major
 constexpr int kBoxBytes = 4 * 32 * 4;
 constexpr int kOffQuick = kOffBox + 2 * kBoxBytes;   // the row's candidates as one unordered list of (bits of p, p in units of 2^-30)
-static_assert(kOffQuick + kQuickCap * 8 <= kRowCtaFixedSmem, "fixed shared-memory area too small");
+constexpr int kOffQsum = kOffQuick + kQuickCap * 8;  // counts and masses at the 32 samples of the search on integer masses
+static_assert(kOffQsum + 256 <= kRowCtaFixedSmem, "fixed shared-memory area too small");
 constexpr int kStripeBytes = 16384;   // 1024 float4 groups: one group per virtual lane
 
 // order-preserving map float -> u32 (no NaN here: inputs are sanitised), so that integer warp reductions serve floats
@@ -148,6 +149,8 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
     unsigned char* cache = smem + pl.off_cache;                          // NC stripes of scaled logits
     uint32_t* s_ncl = reinterpret_cast<uint32_t*>(smem + kOffScal + 8);  // entries of the unordered candidate list
     uint2* qlist = reinterpret_cast<uint2*>(smem + kOffQuick);
+    uint32_t* qsum = reinterpret_cast<uint32_t*>(smem + kOffQsum);
+    if (t < 64) qsum[t] = 0u;
     if (t == 0) {
         *s_idxt = 0;
         *s_token = 0;
@@ -863,12 +866,15 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
             long_lists = __any_sync(FULL, m_max > CR);
             beta_p = __float_as_uint(beta_e / denom);
             if (listed) {
-                // ---- first try: the whole search in warp 0, on integer masses (quick_search)
+                // ---- first try: the whole search on integer masses (quick_sample, quick_settle)
+                __syncthreads();
+                const uint32_t nq = min(*s_ncl, (uint32_t)kQuickCap);
+                quick_sample<WPB>(qlist, nq, pw, lane, qsum);
                 __syncthreads();
                 if (pw == 0) {
                     uint32_t ql, qr, qn;
-                    const int verdict = quick_search<false>(qlist, min(*s_ncl, (uint32_t)kQuickCap), lane, cap + 38, use_cnt, top_k, top_p, beta_p,
-                                                     pmin, pmax, (uint32_t)V, ql, qr, qn);
+                    const int verdict = quick_settle(qlist, nq, lane, qsum, QuickTest(use_cnt, top_k, top_p, cap + 38), top_p, beta_p, pmin,
+                                                     pmax, (uint32_t)V, ql, qr, qn);
                     if (lane == 0) { s_fin[0] = ql; s_fin[1] = qr; s_fin[2] = qn; s_fin[7] = (uint32_t)verdict; }
                 }
                 __syncthreads();

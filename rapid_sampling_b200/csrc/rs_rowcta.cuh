@@ -6,7 +6,7 @@ namespace rs {
 
 struct Params;
 
-constexpr int kRowCtaFixedSmem = 6400;   // scalars, scan totals, the two exchange boxes and the unordered candidate list ahead of the per-lane lists
+constexpr int kRowCtaFixedSmem = 6656;   // scalars, scan totals, the two exchange boxes, the unordered candidate list and its sample sums ahead of the per-lane lists
 
 // How a row-CTA launch lays out its dynamic shared memory.
 struct RowCtaPlan {

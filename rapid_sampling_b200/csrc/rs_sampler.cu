@@ -104,6 +104,8 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     uint64_t* qbar = reinterpret_cast<uint64_t*>(smem + kMiscOff + 40);                       // counts the bytes of the unordered candidate list
     volatile uint32_t* s_quick = reinterpret_cast<volatile uint32_t*>(smem + kMiscOff + 48);  // outcome of the one-warp search: left, right, rounds, verdict
     uint2* qlist = reinterpret_cast<uint2*>(smem + kQuickOff);
+    uint32_t* qsum = reinterpret_cast<uint32_t*>(smem + kQsumOff);
+    if (t < 64) qsum[t] = 0u;      // (ordered by the barrier that follows the mbarriers' set-up)
     // A wait that ran out: the status word (and its host mirror) say so, and this CTA stops producing results --
     // its row reports id -1 and leaves the RNG state and the penalties as they were.
     auto wait_failed = [&]() {
@@ -660,7 +662,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             }
         };
         if (p.quick && ncand <= (uint32_t)kQuickCap) {
-            // ---- first try: the whole search in one warp of every CTA, on integer masses (quick_search).  Every
+            // ---- first try: the whole search on integer masses, in every CTA (quick_sample, quick_settle).  Every
             // CTA gets every candidate of the row: entry k of the list is the same element everywhere (the virtual
             // warps before mine, then the lanes before me), pushed to all CTAs with stores that count their bytes on
             // the destination's barrier.  All CTAs reach the same verdict from the same integers. ----
@@ -684,11 +686,13 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
                 }
             }
             if (C == 1) __syncthreads();
+            else if (!mbar_wait_bounded(qb, 0u, p.wait_polls)) wait_failed();
+            quick_sample<WPC>(qlist, ncand, wl, lane, qsum);
+            __syncthreads();
             if (wl == 0) {
-                if (C > 1 && !mbar_wait_bounded(qb, 0u, p.wait_polls)) wait_failed();
                 uint32_t fl = 0u, fr = 0u, fn = 0u;
-                const int verdict = (*s_fail == 0) ? quick_search<true>(qlist, ncand, lane, cap + 38, use_cnt, top_k, top_p, beta_p, pmin, pmax,
-                                                                  (uint32_t)V, fl, fr, fn)
+                const int verdict = (*s_fail == 0) ? quick_settle(qlist, ncand, lane, qsum, QuickTest(use_cnt, top_k, top_p, cap + 38), top_p,
+                                                                  beta_p, pmin, pmax, (uint32_t)V, fl, fr, fn)
                                                    : 0;
                 if (lane == 0) { s_quick[0] = fl; s_quick[1] = fr; s_quick[2] = fn; s_quick[3] = (uint32_t)verdict; }
             }

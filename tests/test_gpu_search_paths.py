@@ -53,3 +53,14 @@ def test_rows_of_which_nothing_is_cut_off(abi, mode, kind, B, V, temp):
     if mode in (0, 4):
         pen = torch.rand(B, V, generator=torch.Generator().manual_seed(1)) * 0.5
         check_against_oracle(abi, make_logits(kind, B, V, 12, torch), 6, temp, -1, 1.0, mode, pen=pen)
+
+
+@pytest.mark.parametrize("mode", [2, 3, 4])
+@pytest.mark.parametrize("kind,V,k,p", [("normal3", 4, -1, 0.5), ("uniform", 28, 5, 0.9), ("coarse", 64, -1, 0.6), ("equal", 508, 40, 0.3),
+                                        ("uniform", 512, -1, 0.95), ("coarse", 512, 100, 1.0), ("uniform", 516, 200, 0.99),
+                                        ("peaked", 50304, 1, 1.0), ("normal3", 100256, 50, 1e-7), ("coarse", 32768, 250, 0.9)])
+def test_integer_search_by_rank(abi, mode, kind, V, k, p):
+    """Candidate lists shorter than the sample, of exactly and just over the longest length, made of few distinct values,
+    all equal, cut by the count alone, and a top_p inside the margin of the empty set."""
+    for seed in (1, 2):
+        check_against_oracle(abi, make_logits(kind, 6, V, seed, torch), seed, 0.9, k, p, mode)
