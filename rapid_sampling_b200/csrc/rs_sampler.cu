@@ -355,12 +355,14 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
                 for (int j = 0; j < 8; j++) row.st(s + j, v[j]);
             }
         }
+        // (streaming variant: downwards, so that the second pass, which must go upwards, first finds in L2 what was read last)
 #pragma unroll 8
         for (; s < Kt; s++) {
-            float4 v = bulk_load ? row.ld(s) : ldrow4(s * kLanes + tg);
+            const int k = SMEM ? s : Kt - 1 - s;
+            float4 v = bulk_load ? row.ld(k) : ldrow4(k * kLanes + tg);
             v = scaled4(v, a_scale);
             tmax = fmaxf(fmaxf(fmaxf(tmax, v.x), fmaxf(v.y, v.z)), v.w);
-            if (SMEM) row.st(s, v);
+            if (SMEM) row.st(k, v);
         }
     }
     stamp(2);   // pass 1 done
@@ -392,108 +394,150 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     float beta_e = try_cand ? exp2f(beta_x - mx) : INFINITY;
 
     // ---- pass 2: e = exp2f(x - max), ordered denominator (sampling.cu:560-572); min/max of e;
-    // elements with e >= beta_e are appended, in order, to this lane's candidate list.  When the list
-    // looks too thin to settle the cutoff (not more than top_k strictly above the bound, and about less than
-    // top_p of the mass), the bound is lowered 16-fold and the pass repeated, at most twice. -----------
-    float acc, emin, emax, csum, denom;
-    int nc, ns;   // candidates, and those strictly above the bound
-    bool cand_ok;
+    // elements with e >= beta_e are appended, in order, to this lane's candidate list.  A list that looks too thin to
+    // settle the cutoff (not more than top_k strictly above the bound, and about less than top_p of the mass) is
+    // collected again with a lower bound, at most twice: a pass over the scaled logits without exponentials. -----------
+    float acc = 0.f, emin = INFINITY, emax = -INFINITY, csum = 0.f, denom;
+    int nc = 0, ns = 0;   // candidates, and those strictly above the bound
+    bool cand_ok, enough;
     uint32_t ncand, nstrict;
-    const uint32_t* p2box = nullptr;   // the mailbox of the last second pass: word 4 = candidates of each virtual warp
-    auto pass2 = [&](const bool last) -> bool {
-            acc = 0.f; emin = INFINITY; emax = -INFINITY;
-            nc = 0; ns = 0; csum = 0.f;
-        auto pass2_slot = [&](float4 v) {
-            v.x = exp2f(v.x - mx);
-            v.y = exp2f(v.y - mx);
-            v.z = exp2f(v.z - mx);
-            v.w = exp2f(v.w - mx);
+    const uint32_t* p2box = nullptr;   // the mailbox of the last collection: word 4 = candidates of each virtual warp
+    // How far to lower the bound is read off a histogram of a quarter of the elements below it, in eighths of an octave
+    // (calls whose cutoff a large top_p decides; the others' lists are almost never too thin).  It uses the words that
+    // the search's sample sums need later, and leaves them cleared.
+    const bool want_hist = try_cand && a_top_k >= V && a_top_p > 0.5f && V >= 16384;
+    const float sampled = (float)V4 / (float)(max(V4 >> 12, 1) << 10);      // elements that a sampled one stands for
+    const uint32_t beta_bits = __float_as_uint(beta_e);
+    auto sample1 = [&](float e) {
+        const uint32_t bin = (beta_bits - __float_as_uint(e)) >> 20;      // (an element above the bound: a huge number)
+        if (bin < 64u) atomicAdd(qsum + bin, 1u);
+    };
+    auto append = [&](const float4 v) {
+        append_candidates(v, beta_e, cand + t * 4, L * 4, cap, nc, ns);
+        csum += (v.x >= beta_e ? v.x : 0.f) + (v.y >= beta_e ? v.y : 0.f) + (v.z >= beta_e ? v.z : 0.f) + (v.w >= beta_e ? v.w : 0.f);
+    };
+    auto exp4 = [&](float4 v) { return make_float4(exp2f(v.x - mx), exp2f(v.y - mx), exp2f(v.z - mx), exp2f(v.w - mx)); };
+    // NB groups at a time, with ONE test for candidates per batch: a branch per group would end the basic block
+    // there and leave a lone warp waiting out every dependent instruction of its group.
+    auto pass2_batch = [&](auto& v) {
+        constexpr int NB = sizeof(v) / sizeof(float4);
+        float hi_all = 0.f;
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+            v[j] = exp4(v[j]);
             float em = 0.f;
-            em += v.x; em += v.y; em += v.z; em += v.w;
+            em += v[j].x; em += v[j].y; em += v[j].z; em += v[j].w;
             acc += em;
-            const float hi = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
-            emin = fminf(fminf(emin, fminf(v.x, v.y)), fminf(v.z, v.w));
+            const float lo = fminf(fminf(v[j].x, v[j].y), fminf(v[j].z, v[j].w));
+            const float hi = fmaxf(fmaxf(v[j].x, v[j].y), fmaxf(v[j].z, v[j].w));
+            emin = fminf(emin, lo);
             emax = fmaxf(emax, hi);
-            if (hi >= beta_e) {
-                append_candidates(v, beta_e, cand + t * 4, L * 4, cap, nc, ns);
-                csum += (v.x >= beta_e ? v.x : 0.f) + (v.y >= beta_e ? v.y : 0.f) + (v.z >= beta_e ? v.z : 0.f) +
-                        (v.w >= beta_e ? v.w : 0.f);
-            }
-        };
-        // Four groups at a time, with ONE test for candidates per batch: a branch per group would end the basic block
-        // there and leave a lone warp waiting out every dependent instruction of its group.
-        auto pass2_batch = [&](float4 (&v)[4]) {
-            float hi4 = 0.f;
+            hi_all = fmaxf(hi_all, hi);
+        }
+        if (want_hist && NB == 4) {
+            sample1(v[0].x); sample1(v[0].y); sample1(v[0].z); sample1(v[0].w);
+        }
+        if (hi_all >= beta_e) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                v[j].x = exp2f(v[j].x - mx);
-                v[j].y = exp2f(v[j].y - mx);
-                v[j].z = exp2f(v[j].z - mx);
-                v[j].w = exp2f(v[j].w - mx);
-                float em = 0.f;
-                em += v[j].x; em += v[j].y; em += v[j].z; em += v[j].w;
-                acc += em;
-                const float lo = fminf(fminf(v[j].x, v[j].y), fminf(v[j].z, v[j].w));
-                const float hi = fmaxf(fmaxf(v[j].x, v[j].y), fmaxf(v[j].z, v[j].w));
-                emin = fminf(emin, lo);
-                emax = fmaxf(emax, hi);
-                hi4 = fmaxf(hi4, hi);
-            }
-            if (hi4 >= beta_e) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float hi = fmaxf(fmaxf(v[j].x, v[j].y), fmaxf(v[j].z, v[j].w));
-                    if (hi >= beta_e) {
-                        append_candidates(v[j], beta_e, cand + t * 4, L * 4, cap, nc, ns);
-                        csum += (v[j].x >= beta_e ? v[j].x : 0.f) + (v[j].y >= beta_e ? v[j].y : 0.f) + (v[j].z >= beta_e ? v[j].z : 0.f) +
-                                (v[j].w >= beta_e ? v[j].w : 0.f);
-                    }
-                }
-            }
-        };
+            for (int j = 0; j < NB; j++)
+                if (fmaxf(fmaxf(v[j].x, v[j].y), fmaxf(v[j].z, v[j].w)) >= beta_e) append(v[j]);
+        }
+    };
+    // The row as scaled logits in ascending order, four groups at a time with one test for Inf / NaN products, the rest
+    // one by one.  The streaming variant issues the loads of eight (80 registers) or four groups together (B=32,
+    // V=1048576: this pass 54 -> 33 us).
+    auto for_row = [&](auto&& body) {
+        int s = 0;
         if (SMEM) {
-            int s = 0;
             for (; s + 4 <= Kt; s += 4) {
                 float4 v[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++) v[j] = row.ld(s + j);
-                pass2_batch(v);
+                body(v);
             }
-            for (; s < Kt; s++) pass2_slot(row.ld(s));
+            for (; s < Kt; s++) {
+                float4 v[1] = {row.ld(s)};
+                body(v);
+            }
         } else {
-            // streaming variant: the loads of a group of slots are issued together, then consumed in order
+            const float4* q4p = reinterpret_cast<const float4*>(prow) + tg;
+            auto scale4x4 = [&](float4 (&l)[4], float4 (&q)[4]) {
+                float4 v[4];
+                float probe = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    v[j] = rep ? make_float4((l[j].x - q[j].x) * a_scale, (l[j].y - q[j].y) * a_scale, (l[j].z - q[j].z) * a_scale,
+                                             (l[j].w - q[j].w) * a_scale)
+                               : make_float4(l[j].x * a_scale, l[j].y * a_scale, l[j].z * a_scale, l[j].w * a_scale);
+                    probe += fmaf(v[j].w, 0.f, fmaf(v[j].z, 0.f, fmaf(v[j].y, 0.f, v[j].x * 0.f)));
+                }
+                if (probe != probe) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) v[j] = rep ? scaled4_rep(l[j], q[j], a_scale) : scaled4(l[j], a_scale);
+                }
+                body(v);
+            };
+            if (MORE_REGS && !rep) {
+                for (; s + 8 <= Kt; s += 8) {
+                    float4 l[4], m[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) l[j] = ldrow4((s + j) * kLanes + tg);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) m[j] = ldrow4((s + 4 + j) * kLanes + tg);
+                    scale4x4(l, l);
+                    scale4x4(m, m);
+                }
+            }
             if (rep) {
-                constexpr int G = 4;
-                const float4* q4p = reinterpret_cast<const float4*>(prow) + tg;
-                for (int s0 = 0; s0 < Kt; s0 += G) {
-                    float4 lb[G], qb[G];
-    #pragma unroll
-                    for (int j = 0; j < G; j++) {
-                        if (s0 + j < Kt) {
-                            lb[j] = ldrow4((s0 + j) * kLanes + tg);
-                            qb[j] = __ldcg(q4p + (s0 + j) * kLanes);
-                        }
+                for (; s + 4 <= Kt; s += 4) {
+                    float4 l[4], q[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        l[j] = ldrow4((s + j) * kLanes + tg);
+                        q[j] = __ldcg(q4p + (s + j) * kLanes);
                     }
-    #pragma unroll
-                    for (int j = 0; j < G; j++) {
-                        if (s0 + j < Kt) {
-                            pass2_slot(scaled4_rep(lb[j], qb[j], a_scale));
-                        }
-                    }
+                    scale4x4(l, q);
                 }
             } else {
-                constexpr int G = 8;
-                for (int s0 = 0; s0 < Kt; s0 += G) {
-                    float4 lb[G];
-    #pragma unroll
-                    for (int j = 0; j < G; j++)
-                        if (s0 + j < Kt) lb[j] = ldrow4((s0 + j) * kLanes + tg);
-    #pragma unroll
-                    for (int j = 0; j < G; j++)
-                        if (s0 + j < Kt) pass2_slot(scaled4(lb[j], a_scale));
+                for (; s + 4 <= Kt; s += 4) {
+                    float4 l[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) l[j] = ldrow4((s + j) * kLanes + tg);
+                    scale4x4(l, l);
+                }
+            }
+            if (s < Kt) {      // up to three groups: their loads together, too
+                float4 l[3], q[3];
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    if (s + j < Kt) {
+                        l[j] = ldrow4((s + j) * kLanes + tg);
+                        if (rep) q[j] = __ldcg(q4p + (s + j) * kLanes);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    if (s + j < Kt) {
+                        float4 v[1] = {rep ? scaled4_rep(l[j], q[j], a_scale) : scaled4(l[j], a_scale)};
+                        body(v);
+                    }
                 }
             }
         }
+    };
+    // what a collection found, over the whole row; returns its share of the mass
+    auto judge = [&](const uint32_t* box) -> float {
+        p2box = box;
+        cand_ok = try_cand && (__reduce_add_sync(FULL, bx(box, 3, lane)) == 0u);
+        ncand = __reduce_add_sync(FULL, bx(box, 4, lane));
+        nstrict = __reduce_add_sync(FULL, bx(box, 5, lane));
+        const float mass = warp_tree_sum(__uint_as_float(bx(box, 6, lane))) / denom;   // any order: a forecast only
+        enough = (use_cnt && nstrict > (uint32_t)a_top_k) || mass > a_top_p * 1.001f;
+        return mass;
+    };
+    float cmass;
+    {
+        for_row(pass2_batch);
         stamp(4);   // pass 2 done
         acc = warp_tree_sum(acc);
         emin = warp_min(emin);
@@ -503,31 +547,84 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         csum = warp_tree_sum(csum);
         const uint32_t* box = exchange(Packets<2>(), pick4(__float_as_uint(acc), __float_as_uint(emin), __float_as_uint(emax), overflow),
                                        pick4(wnc, wns, __float_as_uint(csum), 0u), 0u);
-        p2box = box;
         denom = warp_tree_sum(__uint_as_float(bx(box, 0, lane)));  // tree over the 32 warp partials (sampling.cu:29-33)
         emin = warp_min(__uint_as_float(bx(box, 1, lane)));
         emax = warp_max(__uint_as_float(bx(box, 2, lane)));
-        cand_ok = try_cand && (__reduce_add_sync(FULL, bx(box, 3, lane)) == 0u);
-        ncand = __reduce_add_sync(FULL, bx(box, 4, lane));
-        nstrict = __reduce_add_sync(FULL, bx(box, 5, lane));
-        const float cmass = warp_tree_sum(__uint_as_float(bx(box, 6, lane))) / denom;   // any order: a forecast only
-        const bool enough = (use_cnt && nstrict > (uint32_t)a_top_k) || cmass > a_top_p * 1.001f;
-        return !cand_ok || enough || last || !(beta_e > 0.f);
-    };
-    if (!pass2(false)) {
-        // A flat row: the lowered bound would already admit every element.  Either the whole row fits the
-        // candidate buffer (one more pass with no bound at all), or there is no point in trying.
-        const bool all_in = beta_e * 0.0625f <= emin;
+        cmass = judge(box);
+    }
+    for (int attempt = 0; attempt < 2 && cand_ok && !enough && beta_e > 0.f; attempt++) {
+        float lowered = beta_e * 0.0625f;
+        if (attempt == 0 && want_hist) {
+            // The CTAs' histograms as estimates of mass and count between the bound and 1, 2, 3, 5 and 8 octaves below it,
+            // added up over the cluster: the first of these levels that makes up the missing mass, with a margin for the
+            // sampling.  A level that would not fit the lists, or none: the whole row is searched.
+            uint32_t wa = 0u, wb = 0u, wc = 0u;
+            __syncthreads();
+            if (wl == 0) {         // lane l: bins l and l + 32; one octave is eight bins
+                const float n0 = sampled * (float)qsum[lane], n1 = sampled * (float)qsum[lane + 32];
+                const float m0 = n0 * beta_e * exp2f(-0.125f * (float)(lane + 1)), m1 = n1 * beta_e * exp2f(-0.125f * (float)(lane + 33));
+                // running sums over the bins, read off where the levels end
+                const float cm = warp_scan_desc(m0, lane), cn = warp_scan_desc(n0, lane);
+                const float dm = __shfl_sync(FULL, cm, 31) + warp_scan_desc(m1, lane), dn = __shfl_sync(FULL, cn, 31) + warp_scan_desc(n1, lane);
+                auto at = [&](float v, int l) { return __float_as_uint(__shfl_sync(FULL, v, l)); };
+                const uint32_t a0 = at(cm, 7), a1 = at(cm, 15), a2 = at(cm, 23), a3 = at(dm, 7), a4 = at(dm, 31);
+                const uint32_t b0 = at(cn, 7), b1 = at(cn, 15), b2 = at(cn, 23), b3 = at(dn, 7), b4 = at(dn, 31);
+                wa = pick4(a0, a1, a2, a3);
+                wb = pick4(a4, b0, b1, b2);
+                wc = pick4(b3, b4, 0u, 0u);
+            }
+            const uint32_t* box = exchange(Packets<3>(), wa, wb, wc);
+            float word = 0.f;                      // lane k: word k, added up over the CTAs (their first warps)
+            if (lane < 10) {
+#pragma unroll
+                for (int c = 0; c < C; c++) word += __uint_as_float(bx(box, lane, c * WPC));
+            }
+            const float need = fmaxf(a_top_p * 1.002f - cmass, 0.f) * denom * 1.05f;
+            const float room = 0.5f * (float)(cap * kLanes) - (float)ncand;
+            lowered = -1.f;
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                const float mk = __shfl_sync(FULL, word, k), ck = __shfl_sync(FULL, word, 5 + k);
+                const float level = k == 0 ? 0.5f : k == 1 ? 0.25f : k == 2 ? 0.125f : k == 3 ? 0.03125f : 0.00390625f;
+                if (lowered < 0.f && mk >= need) lowered = (ck <= room) ? beta_e * level : 0.f;
+            }
+            if (lowered <= 0.f && V > cap * kLanes) {
+                cand_ok = false;
+                break;
+            }
+            lowered = fmaxf(lowered, 0.f);
+        }
+        // a flat row: the lowered bound would already admit every element.  Either the whole row fits the candidate
+        // buffer (no bound at all), or there is no point in trying.
+        const bool all_in = lowered <= emin;
         if (all_in && V > cap * kLanes) {
             cand_ok = false;
-        } else {
-            beta_e = all_in ? 0.f : beta_e * 0.0625f;
-            if (!pass2(false)) {
-                beta_e *= 0.0625f;
-                pass2(true);
-            }
+            break;
         }
+        beta_e = all_in ? 0.f : lowered;
+        // candidates alone: a compare on x (with slack for the rounding of exp2f) spares the others the exponential
+        nc = 0; ns = 0; csum = 0.f;
+        const float xcut = (beta_e > 1e-35f) ? mx + log2f(beta_e) - 0.01f - fabsf(mx) * 1e-6f : -INFINITY;
+        for_row([&](auto& v) {
+            constexpr int NB = sizeof(v) / sizeof(float4);
+            float hi_all = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < NB; j++) hi_all = fmaxf(hi_all, fmaxf(fmaxf(v[j].x, v[j].y), fmaxf(v[j].z, v[j].w)));
+            if (hi_all >= xcut) {
+#pragma unroll
+                for (int j = 0; j < NB; j++)
+                    if (fmaxf(fmaxf(v[j].x, v[j].y), fmaxf(v[j].z, v[j].w)) >= xcut) {
+                        const float4 e = exp4(v[j]);
+                        if (fmaxf(fmaxf(e.x, e.y), fmaxf(e.z, e.w)) >= beta_e) append(e);
+                    }
+            }
+        });
+        const unsigned overflow = __any_sync(FULL, nc > cap) ? 1u : 0u;
+        const uint32_t wnc = __reduce_add_sync(FULL, (uint32_t)nc), wns = __reduce_add_sync(FULL, (uint32_t)ns);
+        csum = warp_tree_sum(csum);
+        cmass = judge(exchange(Packets<2>(), pick4(0u, 0u, 0u, overflow), pick4(wnc, wns, __float_as_uint(csum), 0u), 0u));
     }
+    if (want_hist && wl == 0) qsum[lane] = qsum[lane + 32] = 0u;
     // division is monotone, so the row's min/max probability are the quotients of min/max e
     const float pmin = emin / denom, pmax = emax / denom;
     if (p.dbg_probs) {   // test instrumentation: the probabilities of the whole row
@@ -548,119 +645,134 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     const float top_p = a_top_p;
     uint32_t left = 0, right = 0, rounds = 0, n_eval = 0;
     uint32_t path = 1;
-    uint32_t conv_cnt = 0, conv_left_cnt = 0;   // counts at `right` / `left` and ordered mass at `right` on return
-    float conv_mass = 0.f;
-
-    // The reference's loop, replayed with the same pivots and the same decisions.  `lane_eval` returns this
-    // lane's ordered masses / counts for four pivots over whatever list the caller searches.
+    // The reference's loop, replayed with the same pivots and the same decisions.  Its test at a pivot u depends only on
+    // the set {p >= u}, and both its count and its ordered fp32 mass can only grow as u falls (a rounded sum of the same
+    // association does not decrease when a term >= 0 takes the place of a zero).  So one evaluated point answers every
+    // pivot on its far side: points below `za` are known to exceed top_k or top_p, points from `zb` on pass, points in
+    // [e0, e1] do neither.  Pivots inside the unknown zone [za, zb) are settled by evaluating four points of our own
+    // choice, placed by interpolation on mass and count, which close in on the boundary much faster than the pivots'
+    // quartering: about 6 evaluations instead of 12 to 15 (B=4, V=131072, flat: 49.6 -> 45.0 us a call).
     //  * clamp (candidate list only): every probability above beta_p is on the list, so a pivot above beta_p
     //    sees exactly the elements the reference sees.  A pivot u <= beta_p is not evaluated; instead the set
     //    {p > beta_p} is (pivot u*, the next float after beta_p): if it already holds more than top_k elements
     //    or more than top_p mass, so does the larger set {p >= u}, hence the reference's test at u fails and
     //    its carried state keeps the loop going -- all it uses these values for.  Otherwise: not valid.
-    //  * bounds (candidate list only): once every element strictly inside (left, right) has one and the same
-    //    value v, the remaining rounds need no data: a pivot equal to `left` selects the set of `left`, a pivot
-    //    in (left, v] the set {p >= v}, a pivot above v the set of `right`; they are replayed arithmetically.
-    auto run_search = [&](auto&& lane_eval, const bool clamp, const uint32_t beta_p, const bool sure_cnt,
-                          const uint32_t n_above) -> bool {
+    //  * bounds: the smallest and largest element inside the zone move its ends up to them without an evaluation.
+    // `lane_eval(f, keep, lo, hi, cnt_keep, ...)` returns this lane's ordered masses and counts at four points, and the
+    // bounds of its elements in [lo, hi); elements below `keep` (there are cnt_keep from it on) will not be asked for again.
+    auto run_search = [&](auto&& lane_eval, const bool clamp, const uint32_t beta_p, const bool sure_cnt) -> bool {
         const uint32_t ustar = clamp ? beta_p + 1u : 0u;
         left = __float_as_uint(pmin);
         right = __float_as_uint(pmax) + 1u;
         rounds = 0;
-        uint32_t cnt_x = (uint32_t)V, cnt_r = 0u;   // counts at left / at right
-        float mass_x = 1.0f, mass_r = 0.f;
-        bool frozen = false, valid = true;
-        uint32_t v_bits = 0, cnt_v = 0;
-        float mass_v = 0.f;
-        while (rounds < 64u) {
-            const bool go = use_cnt ? (cnt_x > top_k || mass_x > top_p) : (mass_x > top_p);
-            if (!(go && left < right - 1u)) break;
-            rounds++;
+        uint32_t za = max(left, ustar) + ((clamp && sure_cnt) ? 1u : 0u), zb = right;
+        uint32_t e0 = 1u, e1 = 0u;                        // none yet
+        uint32_t cnt_a = (uint32_t)V, cnt_b = 0u;         // of the sets at za - 1 and zb (estimates until evaluated)
+        float mass_a = 1.0f, mass_b = 0.f;
+        const bool odd = zb <= za || !(0.f < top_p);      // not even the empty set is known to pass
+        if (odd) zb = 0x7f800000u;
+        int n_since = 0;                                  // evaluations of this search
+        bool slow = false;
+        bool go = (use_cnt && (uint32_t)V > top_k) || 1.0f > top_p;
+        while (go && left < right - 1u && rounds < 64u) {
             const uint32_t pz = (left + right) >> 1, py = (left + pz) >> 1, pw = (pz + right) >> 1;
-            const uint32_t pv[3] = {py, pz, pw};
-            uint32_t cnt[4];
-            float mass[4];
-            if (clamp && sure_cnt && pw <= beta_p) {
-                // All three pivots lie at or below the bound, and more than top_k elements are known to lie
-                // strictly above it: every test fails, the lower end moves to the last pivot, no data is needed.
-                left = pw;
-                cnt_x = n_above;
-                mass_x = 0.f;
+            // 2 exceeds, 1 neither, 0 passes, -1 unknown
+            auto known = [&](uint32_t u) -> int {
+                u = max(u, ustar);
+                return u < za ? 2 : u >= zb ? 0 : (u >= e0 && u <= e1) ? 1 : -1;
+            };
+            const int c0 = known(py), c1 = known(pz), c2 = known(pw);
+            // the reference asks from the lowest pivot up and stops at the first that passes
+            const bool open0 = c0 < 0, open1 = c0 > 0 && c1 < 0, open2 = c0 > 0 && c1 > 0 && c2 < 0;
+            if (open0 || open1 || open2) {
+                const uint32_t ask = max(open0 ? py : open1 ? pz : pw, ustar);
+                uint32_t lo = za, hi = zb;               // the part of the zone that holds the asked point
+                const bool some = e0 <= e1;
+                if (some && ask > e1) lo = e1 + 1u;
+                if (some && ask < e0) hi = e0;
+                const uint32_t w = hi - lo;
+                uint32_t u[4];
+                if (w <= 4u) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) u[i] = min(lo + (uint32_t)i, hi - 1u);
+                } else {
+                    const float fw = (float)w;
+                    float at = 0.5f, d0 = 0.1f, d1 = 0.3f;              // .2 .4 .6 .8
+                    if (n_since > 0 && !slow && !some) {
+                        const float n_in = fmaxf((float)cnt_a - (float)cnt_b, 1.f);
+                        const float tm = __fdividef(mass_a - top_p, mass_a - mass_b);
+                        const float tc = use_cnt ? __fdividef((float)cnt_a - (float)top_k + 0.5f, n_in) : 0.f;
+                        at = fminf(fmaxf(fmaxf(tm, tc), 0.f), 1.f);
+                        d1 = fminf(fmaxf(n_since == 1 ? 0.12f : n_since == 2 ? 0.06f : 0.03f, rsqrtf(n_in)), 0.3f);
+                        d0 = 0.33f * d1;
+                        at = fminf(fmaxf(at, d0), 1.f - d0);
+                    }
+                    const float q[4] = {at - d1, at - d0, at + d0, at + d1};
+#pragma unroll
+                    for (int i = 0; i < 4; i++) u[i] = min(lo + (uint32_t)(fminf(fmaxf(q[i], 0.f), 1.f) * fw), hi - 1u);
+                    if (some || n_since >= 12) u[1] = ask;
+                }
+                n_eval++;
+                n_since++;
+                const float f[4] = {__uint_as_float(u[0]), __uint_as_float(u[1]), __uint_as_float(u[2]), __uint_as_float(u[3])};
+                float m[4], mass[4];
+                uint32_t cnt[4], c01, c23, mn, mxv, vmin, vmax;
+                lane_eval(f, za > 0u ? za - 1u : 0u, za, zb, cnt_a, m, c01, c23, mn, mxv);
+                totals(m, c01, c23, mn, mxv, cnt, mass, vmin, vmax);
+                const uint32_t za_old = za, w_old = zb - za;
+                // the highest point that exceeds, the lowest that passes
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const bool exc = (use_cnt && cnt[i] > top_k) || mass[i] > top_p;
+                    const bool pass = (!use_cnt || cnt[i] < top_k) && mass[i] < top_p;
+                    if (exc) {
+                        if (u[i] >= za) { za = u[i] + 1u; cnt_a = cnt[i]; mass_a = mass[i]; }
+                    } else if (pass) {
+                        if (u[i] < zb) { zb = u[i]; cnt_b = cnt[i]; mass_b = mass[i]; }
+                    } else if (e0 > e1) {
+                        e0 = e1 = u[i];
+                    } else {
+                        e0 = min(e0, u[i]);
+                        e1 = max(e1, u[i]);
+                    }
+                }
+                // every element that was inside the zone lies in [vmin, vmax] (none: vmin > vmax)
+                if (!odd && e0 > e1) {
+                    if (vmin > vmax) zb = za;                         // the sets of the zone are all the set at zb
+                    else if (vmax + 1u < zb) zb = max(vmax + 1u, za);
+                    if (za > za_old && vmin >= za && vmin < zb) za = vmin + 1u;   // {>= vmin} is the set at za - 1
+                }
+                slow = (zb - za) > (w_old >> 2);
                 continue;
             }
-            if (!frozen) {
-                n_eval++;
-                const float f[4] = {__uint_as_float(max(py, ustar)), __uint_as_float(max(pz, ustar)),
-                                    __uint_as_float(max(pw, ustar)), __uint_as_float(max(left + 1u, ustar))};
-                float m[4];
-                uint32_t c01, c23, mn, mxv, vmin, vmax;
-                lane_eval(f, left, right, cnt_x, m, c01, c23, mn, mxv);
-                totals(m, c01, c23, mn, mxv, cnt, mass, vmin, vmax);
-                if (clamp && left >= beta_p && vmin >= vmax) {   // one distinct value inside (none: vmin > vmax)
-                    frozen = true;
-                    v_bits = (vmin == vmax) ? vmin : left;
-                    cnt_v = cnt[3];      // the set {p >= left + 1} is {p >= v}
-                    mass_v = mass[3];
-                }
+            if (clamp && ((py <= beta_p && c0 < 2) || (c0 > 0 && pz <= beta_p && c1 < 2) || (c0 > 0 && c1 > 0 && pw <= beta_p && c2 < 2)))
+                return false;
+            rounds++;
+            if (c0 == 0) {
+                right = py;
+            } else if (c1 == 0) {
+                left = py; right = pz; go = c0 == 2;
+            } else if (c2 == 0) {
+                left = pz; right = pw; go = c1 == 2;
             } else {
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const bool at_left = (pv[i] == left), le_v = (pv[i] <= v_bits);
-                    cnt[i] = at_left ? cnt_x : le_v ? cnt_v : cnt_r;
-                    mass[i] = at_left ? mass_x : le_v ? mass_v : mass_r;
-                }
+                left = pw; go = c2 == 2;
             }
-            // the three tests and the bracket update, written with selects: this is the critical path of every round
-            bool ok[3], bad = false;
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                const bool below = clamp && pv[i] <= beta_p;
-                const bool exceeds = (use_cnt && cnt[i] > top_k) || mass[i] > top_p;
-                const bool pass = (!use_cnt || cnt[i] < top_k) && mass[i] < top_p;
-                ok[i] = !below && pass;
-                bad = bad || (below && !exceeds);
-            }
-            if (bad) { valid = false; break; }
-            const bool s0 = ok[0], s1 = !s0 && ok[1], s2 = !s0 && !s1 && ok[2];   // none: the bracket's upper part
-            const uint32_t nl = s0 ? left : s1 ? py : s2 ? pz : pw;
-            const uint32_t nr = s0 ? py : s1 ? pz : s2 ? pw : right;
-            const uint32_t ncx = s0 ? cnt_x : s1 ? cnt[0] : s2 ? cnt[1] : cnt[2];
-            const float nmx = s0 ? mass_x : s1 ? mass[0] : s2 ? mass[1] : mass[2];
-            const uint32_t ncr = s0 ? cnt[0] : s1 ? cnt[1] : s2 ? cnt[2] : cnt_r;
-            const float nmr = s0 ? mass[0] : s1 ? mass[1] : s2 ? mass[2] : mass_r;
-            left = nl; right = nr; cnt_x = ncx; mass_x = nmx; cnt_r = ncr; mass_r = nmr;
         }
-        conv_cnt = cnt_r;
-        conv_mass = mass_r;
-        conv_left_cnt = cnt_x;
-        return valid && (!clamp || left > beta_p);
+        return !clamp || left > beta_p;
     };
 
     float gtp = 0.f;         // this lane's mass above the threshold, its ties with it, its count above
     uint32_t eqk = 0, gtk = 0;
-    bool done = false;
-    int quick = 0;           // outcome of the one-warp search on integer masses: 0 not settled that way, 1 settled, 2 list too short
+    int quick = 0;           // outcome of the search on integer masses: 0 not settled that way, 1 settled, 2 list too short
+    // The list that is searched: the lane's candidates, or all of its elements; both lie in float4 slots, `lstride` apart.
+    float4* lbase = reinterpret_cast<float4*>(cand) + t;
+    int lstride = L, n = cand_ok ? min(nc, cap) : 0;
+    uint32_t beta_p = 0u;
     if (cand_ok) {
-        // ===== candidate list: a few elements per lane at most =====
-        const int m_own = min(nc, cap);
+        const int m_own = n;
         for (int i = 0; i < m_own; i++) cand_at(i) = cand_at(i) / denom;
-        const uint32_t beta_p = __float_as_uint(beta_e / denom);
-        auto cand_eval = [&](const float (&f)[4], uint32_t lo, uint32_t hi, uint32_t, float (&m)[4], uint32_t& c01,
-                             uint32_t& c23, uint32_t& mn, uint32_t& mxv) {
-            m[0] = m[1] = m[2] = m[3] = 0.f;
-            c01 = c23 = 0u;
-            mn = 0xffffffffu;
-            mxv = 0u;
-            for (int i = 0; i < m_own; i++) {
-                const float q = cand_at(i);
-                const uint32_t qb = __float_as_uint(q);
-                if (q >= f[0]) { c01 += 1u; m[0] += q; }
-                if (q >= f[1]) { c01 += 0x10000u; m[1] += q; }
-                if (q >= f[2]) { c23 += 1u; m[2] += q; }
-                if (q >= f[3]) { c23 += 0x10000u; m[3] += q; }
-                if (qb > lo && qb < hi) { mn = min(mn, qb); mxv = max(mxv, qb); }
-            }
-        };
+        for (int i = m_own; i < ((m_own + 3) & ~3); i++) cand_at(i) = -1.f;     // no pivot admits it
+        beta_p = __float_as_uint(beta_e / denom);
         if (p.quick && ncand <= (uint32_t)kQuickCap) {
             // ---- first try: the whole search on integer masses, in every CTA (quick_sample, quick_settle).  Every
             // CTA gets every candidate of the row: entry k of the list is the same element everywhere (the virtual
@@ -687,6 +799,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             }
             if (C == 1) __syncthreads();
             else if (!mbar_wait_bounded(qb, 0u, p.wait_polls)) wait_failed();
+            if (want_hist) __syncthreads();      // the sample sums have been cleared
             quick_sample<WPC>(qlist, ncand, wl, lane, qsum);
             __syncthreads();
             if (wl == 0) {
@@ -700,113 +813,103 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             quick = (int)s_quick[3];
             if (quick == 1) { left = s_quick[0]; right = s_quick[1]; rounds = s_quick[2]; }
         }
-        if (quick == 2) {
-            // the list cannot settle the cutoff: the whole row is searched
-        } else if (ncand <= 4096u) {
-            done = (quick == 1) ? true : run_search(cand_eval, true, beta_p, use_cnt && nstrict > top_k, nstrict);
-            if (done) {
-                path = 0;
-                const float thr = __uint_as_float(left);
-                for (int i = 0; i < m_own; i++) {
-                    const float q = cand_at(i);
-                    if (q == thr) eqk++;
-                    if (q > thr) { gtk++; gtp += q; }
-                }
-            }
-        } else {
-            // Long lists (flat rows whose lowered bound took in much of the row): the buffer has the slab's
-            // [slot][lane] float4 layout, so it is searched like a slab -- vector loads, and elements below
-            // `left` dropped in place once the bracket has risen above the bound.
-            for (int i = m_own; i < ((m_own + 3) & ~3); i++) cand_at(i) = -1.f;
-            Row<C, true> crow;
-            crow.slab = reinterpret_cast<float4*>(cand);
-            crow.t = t;
-            crow.tg = tg;
-            int n = m_own;
-            uint32_t list_total = ncand, list_left = 0u;
-            auto cand_slab_eval = [&](const float (&f)[4], uint32_t lo, uint32_t, uint32_t cnt_lo, float (&m)[4], uint32_t& c01,
-                                      uint32_t& c23, uint32_t& mn, uint32_t& mxv) {
-                mn = 0u;
-                mxv = 1u;   // bounds are not tracked for long lists
-                const bool compact = (lo != list_left) && (lo > beta_p) && (cnt_lo * 2u <= list_total);
-                if (compact) {
-                    slab_pass<C, true, true>(crow, n, f, __uint_as_float(lo), m, c01, c23);
-                    list_total = cnt_lo;
-                    list_left = lo;
-                } else {
-                    slab_pass<C, true, false>(crow, n, f, 0.f, m, c01, c23);
-                }
-            };
-            done = run_search(cand_slab_eval, true, beta_p, use_cnt && nstrict > top_k, nstrict);
-            if (done) {
-                path = 0;
-                const float thr = __uint_as_float(left);
-                for (int i = 0; i < n; i++) {
-                    const float q = cand_at(i);
-                    if (q == thr) eqk++;
-                    if (q > thr) { gtk++; gtp += q; }
-                }
-            }
-        }
     }
-    if (!done && emin == emax) {
-        // Every element has the same probability: the reference's loop never starts (left = pmin, right = left + 1),
-        // the threshold is that probability and the whole row ties with it.  No pass is needed.
-        left = __float_as_uint(pmin);
-        right = left + 1u;
-        eqk = (uint32_t)(Kt * 4);
-    } else if (!done && top_p >= 1.0f && (!use_cnt || top_k >= (uint32_t)V)) {
-        // Nothing is cut off: the reference's loop never starts (sampling.cu:598) and leaves left = pmin.  What is left
-        // of its work is the recount, so the probabilities are summed as they are computed and never stored (B=256,
-        // V=151936: 155.7 -> 100.9 us; the scratch row cost a write and a read of 155 MB and the general division).
-        left = __float_as_uint(pmin);
-        right = __float_as_uint(pmax) + 1u;
-        const float inv = __frcp_rn(denom);
+    // Candidates first, then the whole row, through one copy of the search: this code runs once or twice per call, so its
+    // size in the instruction cache costs as much as its arithmetic.
+    for (int attempt = (cand_ok && quick != 2) ? 0 : 1; attempt < 2; attempt++) {
+        const bool whole = attempt == 1;
+        uint32_t list_total = ncand, list_left = 0u;     // live elements; the list holds all that are >= list_left
+        if (whole) {
+            left = __float_as_uint(pmin);
+            if (emin == emax) {
+                // Every element has the same probability: the reference's loop never starts (left = pmin, right = left + 1),
+                // the threshold is that probability and the whole row ties with it.  No pass is needed.
+                right = left + 1u;
+                eqk = (uint32_t)(Kt * 4);
+                break;
+            }
+            const float inv = __frcp_rn(denom);
+            if (top_p >= 1.0f && (!use_cnt || top_k >= (uint32_t)V)) {
+                // Nothing is cut off: the reference's loop never starts (sampling.cu:598) and leaves left = pmin.  What is
+                // left of its work is the recount, so the probabilities are summed as they are computed and never stored
+                // (B=256, V=151936: 155.7 -> 100.9 us; the scratch row cost a write and a read of 155 MB and the general
+                // division).
+                right = __float_as_uint(pmax) + 1u;
 #pragma unroll 4
-        for (int s = 0; s < Kt; s++) add_open(prob4(xload(s), mx, denom, inv), pmin, gtp, eqk);
-        gtk = (uint32_t)(Kt * 4) - eqk;
-    } else if (!done) {
-        // ===== whole row: pass 3, p = exp2f(x - max) / denom (sampling.cu:573-590), in place; then the search
-        // over every lane's full list, dropping elements below `left` as the bracket rises =====
+                for (int s = 0; s < Kt; s++) add_open(prob4(xload(s), mx, denom, inv), pmin, gtp, eqk);
+                gtk = (uint32_t)(Kt * 4) - eqk;
+                break;
+            }
+            // pass 3, p = exp2f(x - max) / denom (sampling.cu:573-590), in place
 #pragma unroll (SMEM ? 2 : 4)
-        for (int s = 0; s < Kt; s++) {
-            float4 v = xload(s);
-            v.x = exp2f(v.x - mx) / denom;
-            v.y = exp2f(v.y - mx) / denom;
-            v.z = exp2f(v.z - mx) / denom;
-            v.w = exp2f(v.w - mx) / denom;
-            row.st(s, v);
+            for (int s = 0; s < Kt; s++) row.st(s, prob4(xload(s), mx, denom, inv));
+            lbase = row.slab + (SMEM ? t : tg);
+            lstride = SMEM ? L : kLanes;
+            n = Kt * 4;
+            list_total = (uint32_t)V;
+            list_left = left;
         }
-        int n = Kt * 4;                      // live elements of this lane's list
-        uint32_t list_total = (uint32_t)V;   // live elements over the whole row
-        uint32_t list_left = __float_as_uint(pmin);   // the list holds exactly the elements >= list_left
-        auto slab_eval = [&](const float (&f)[4], uint32_t lo, uint32_t, uint32_t cnt_lo, float (&m)[4], uint32_t& c01,
+        auto list_eval = [&](const float (&f)[4], uint32_t keep, uint32_t lo, uint32_t hi, uint32_t cnt_keep, float (&m)[4], uint32_t& c01,
                              uint32_t& c23, uint32_t& mn, uint32_t& mxv) {
-            mn = 0u;
-            mxv = 1u;   // bounds are not tracked here
-            const bool compact = (lo != list_left) && (cnt_lo * 2u <= list_total);
-            if (compact) {
-                slab_pass<C, SMEM, true>(row, n, f, __uint_as_float(lo), m, c01, c23);
-                list_total = cnt_lo;
-                list_left = lo;
-            } else {
-                slab_pass<C, SMEM, false>(row, n, f, 0.f, m, c01, c23);
+            if (keep != list_left && cnt_keep * 2u <= list_total) {
+                // half of the list will not be asked for again: dropped in place, order preserved
+                const float kf = __uint_as_float(keep);
+                int q = 0;
+                for (int i = 0; i < n; i += 4) {
+                    const float4 v = lbase[(i >> 2) * lstride];
+                    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        if (e[j] >= kf) {
+                            reinterpret_cast<float*>(lbase + (q >> 2) * lstride)[q & 3] = e[j];
+                            q++;
+                        }
+                    }
+                }
+                n = q;
+                for (; q & 3; q++) reinterpret_cast<float*>(lbase + (q >> 2) * lstride)[q & 3] = -1.f;
+                list_total = cnt_keep;
+                list_left = keep;
+            }
+            mn = 0xffffffffu;
+            mxv = 0u;
+            m[0] = m[1] = m[2] = m[3] = 0.f;
+            c01 = c23 = 0u;
+#pragma unroll 2
+            for (int i = 0; i < n; i += 4) {
+                const float4 v = lbase[(i >> 2) * lstride];
+                const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float q = e[j];
+                    const uint32_t qb = __float_as_uint(q);
+                    const bool in = qb >= lo && qb < hi;          // (the padding's bits are above any hi)
+                    c01 += (q >= f[0] ? 1u : 0u) + (q >= f[1] ? 0x10000u : 0u);
+                    c23 += (q >= f[2] ? 1u : 0u) + (q >= f[3] ? 0x10000u : 0u);
+                    m[0] += q >= f[0] ? q : 0.f;                  // (adding zero changes no sum of terms >= 0)
+                    m[1] += q >= f[1] ? q : 0.f;
+                    m[2] += q >= f[2] ? q : 0.f;
+                    m[3] += q >= f[3] ? q : 0.f;
+                    mn = min(mn, in ? qb : 0xffffffffu);
+                    mxv = max(mxv, in ? qb : 0u);
+                }
             }
         };
-        run_search(slab_eval, false, 0u, false, 0u);
+        if (quick != 1 && !run_search(list_eval, !whole, beta_p, !whole && use_cnt && nstrict > top_k) && !whole) continue;
         // recount at the threshold (sampling.cu:657-680)
         const float thr = __uint_as_float(left);
-        const int slots = (n + 3) >> 2;
-#pragma unroll 2
-        for (int s = 0; s < slots; s++) {
-            const float4 v = row.ld(s);
+        for (int i = 0; i < n; i += 4) {
+            const float4 v = lbase[(i >> 2) * lstride];
             const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                if (e[j] == thr) eqk++;
-                if (e[j] > thr) { gtk++; gtp += e[j]; }
+                eqk += e[j] == thr ? 1u : 0u;
+                gtk += e[j] > thr ? 1u : 0u;
+                gtp += e[j] > thr ? e[j] : 0.f;
             }
         }
+        path = whole ? 1u : 0u;
+        break;
     }
     stamp(6);   // search and recount done
     const bool early_exit = left < right - 1u;
@@ -816,13 +919,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     // same tree value as the butterfly, and the warp values are then added in warp order.
     float sgtp;
     uint32_t seqk, sgtk;
-    if (path == 0 && !early_exit && quick != 1) {
-        // The bracket closed (right == left + 1): the set at `right` is exactly {p > threshold}, and its count
-        // and ordered mass were carried along by the search; the ties are the rest of the set at `left`.
-        sgtp = conv_mass;
-        sgtk = conv_cnt;
-        seqk = conv_left_cnt - conv_cnt;
-    } else {
+    {
         const float m[4] = {gtp, 0.f, 0.f, 0.f};
         uint32_t cnt[4], d0, d1;
         float mass[4];

@@ -64,3 +64,21 @@ def test_integer_search_by_rank(abi, mode, kind, V, k, p):
     all equal, cut by the count alone, and a top_p inside the margin of the empty set."""
     for seed in (1, 2):
         check_against_oracle(abi, make_logits(kind, 6, V, seed, torch), seed, 0.9, k, p, mode)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])        # the planner's choice, whole row only, streaming, on-chip
+@pytest.mark.parametrize("kind,B,V,temp,k,p", [("normal3", 2, 16384, 1.0, -1, 0.9), ("normal3", 3, 16388, 1.0, -1, 0.99),
+                                               ("peaked", 130, 50304, 1.0, -1, 0.95), ("uniform", 2, 131072, 1.0, -1, 0.5),
+                                               ("uniform", 4, 20484, 0.7, -1, 0.999999), ("normal3", 3, 65536, 0.8, 1000, 0.95),
+                                               ("coarse", 3, 50304, 0.9, 3000, 0.99), ("coarse", 2, 32768, 1.0, -1, 0.6),
+                                               ("special", 3, 50304, 1.3, 700, 0.9), ("normal3", 2, 65536, 0.02, 300, 0.9999),
+                                               ("uniform4", 2, 8192, 1.0, 8191, 1.0), ("normal3", 2, 16384, 1.0, -1, 1e-46),
+                                               ("equal", 2, 32768, 1.0, 500, 0.9)])
+def test_wide_kept_sets(abi, mode, kind, B, V, temp, k, p):
+    """Cutoffs far down the row: lists collected again under a bound read off the histogram, long lists, and whole rows, all
+    searched by evaluating points of the kernel's own choice; ties, counts met exactly, zero probabilities, and a top_p
+    that is zero in fp32."""
+    check_against_oracle(abi, make_logits(kind, B, V, 21, torch), 9, temp, k, p, mode)
+    if B <= 4 and mode != 1:
+        pen = torch.rand(B, V, generator=torch.Generator().manual_seed(2)) * 0.5
+        check_against_oracle(abi, make_logits(kind, B, V, 22, torch), 10, temp, k, p, mode, pen=pen)
