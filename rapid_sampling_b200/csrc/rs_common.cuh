@@ -137,10 +137,11 @@ __device__ __forceinline__ void slab_pass(const Row<C, SMEM>& row, int& n, const
 struct QuickTest {       // the three possible outcomes of the reference's tests at a set of count c and mass m
     bool use_cnt;
     uint32_t top_k, tp_lo, tp_hi, margin;
-    __device__ __forceinline__ QuickTest(bool uc, uint32_t k, float top_p, int depth) {
+    // depth: additions on the longest path of the reference's sum; cap: longest list (half a unit of rounding per entry)
+    __device__ __forceinline__ QuickTest(bool uc, uint32_t k, float top_p, int depth, int cap = kQuickCap) {
         use_cnt = uc;
         top_k = k;
-        margin = (uint32_t)(depth * 66 + kQuickCap / 2 + 8);
+        margin = (uint32_t)(depth * 66 + cap / 2 + 8);
         tp_lo = __float2uint_rd(top_p * 1073741824.f);
         tp_hi = __float2uint_ru(top_p * 1073741824.f);
     }
@@ -192,14 +193,23 @@ __device__ __forceinline__ int quick_settle(uint2* list, const uint32_t n, const
         // what lies between: compacted to the front of the list (a place is written only after it has been read)
         const uint32_t lo = max(x2, beta_p);
         uint32_t q = 0u;
-        for (uint32_t i0 = 0u; i0 < nz; i0 += 32u) {
-            const uint32_t i = i0 + (uint32_t)lane;
-            const uint2 e = (i < nz) ? list[i] : make_uint2(0u, 0u);
-            const bool in = e.x > lo && e.x < x0;
-            const unsigned b = __ballot_sync(FULLW, in);
+        for (uint32_t i0 = 0u; i0 < nz; i0 += 128u) {
+            uint2 e[4];
+            unsigned b[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint32_t i = i0 + (uint32_t)(32 * j + lane);
+                e[j] = (i < nz) ? list[i] : make_uint2(0u, 0u);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) b[j] = __ballot_sync(FULLW, e[j].x > lo && e[j].x < x0);
             __syncwarp();
-            if (in) list[q + (uint32_t)__popc(b & ((1u << lane) - 1u))] = e;
-            q += (uint32_t)__popc(b);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if ((b[j] >> lane) & 1u) list[q + (uint32_t)__popc(b[j] & ((1u << lane) - 1u))] = e[j];
+                q += (uint32_t)__popc(b[j]);
+            }
+            __syncwarp();
         }
         __syncwarp();
         nz = q;

@@ -148,7 +148,11 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
     unsigned char* ring = smem + pl.off_ring;                            // D stages of pl.stage_bytes
     unsigned char* cache = smem + pl.off_cache;                          // NC stripes of scaled logits
     uint32_t* s_ncl = reinterpret_cast<uint32_t*>(smem + kOffScal + 8);  // entries of the unordered candidate list
-    uint2* qlist = reinterpret_cast<uint2*>(smem + kOffQuick);
+    // the unordered candidate list: without penalties the copy stages are idle during the search and take twice the entries
+    // (B=160, V=100256, top_k 100: lists of 220 to 630; those above 512 went to the exact search, 12 us more for such a row)
+    constexpr uint32_t kListCap = REP ? kQuickCap : 2 * kQuickCap;
+    static_assert(REP || kListCap * 8 <= D * kStripeBytes / NH, "the list must fit the copy stages");
+    uint2* qlist = reinterpret_cast<uint2*>(REP ? smem + kOffQuick : ring);
     uint32_t* qsum = reinterpret_cast<uint32_t*>(smem + kOffQsum);
     if (t < 64) qsum[t] = 0u;
     if (t == 0) {
@@ -837,7 +841,7 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
                 mine += m_own[j];
             }
             // a place for this thread's entries in the row's unordered list (short lists only)
-            const bool listed = p.quick && ncand <= (uint32_t)kQuickCap;
+            const bool listed = p.quick && ncand <= kListCap;
             uint32_t at = 0u;
             if (listed) {
                 uint32_t incl = (uint32_t)mine;
@@ -868,12 +872,12 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
             if (listed) {
                 // ---- first try: the whole search on integer masses (quick_sample, quick_settle)
                 __syncthreads();
-                const uint32_t nq = min(*s_ncl, (uint32_t)kQuickCap);
+                const uint32_t nq = min(*s_ncl, kListCap);
                 quick_sample<WPB>(qlist, nq, pw, lane, qsum);
                 __syncthreads();
                 if (pw == 0) {
                     uint32_t ql, qr, qn;
-                    const int verdict = quick_settle(qlist, nq, lane, qsum, QuickTest(use_cnt, top_k, top_p, cap + 38), top_p, beta_p, pmin,
+                    const int verdict = quick_settle(qlist, nq, lane, qsum, QuickTest(use_cnt, top_k, top_p, cap + 38, kListCap), top_p, beta_p, pmin,
                                                      pmax, (uint32_t)V, ql, qr, qn);
                     if (lane == 0) { s_fin[0] = ql; s_fin[1] = qr; s_fin[2] = qn; s_fin[7] = (uint32_t)verdict; }
                 }
