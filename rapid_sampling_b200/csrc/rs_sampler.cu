@@ -317,15 +317,24 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     // ---- pass 1: x = sanitised scaled logit (sampling.cu:208-227, :547-559); row max; and this
     // thread's own maximum, from which a lower bound for the cutoff is derived below -------------
     float tmax = -INFINITY;
+    // Penalties are zero but for the tokens a context has used: one bit per group (the first 64) notes where this lane's are
+    // not all +0.  The other groups are neither read again nor rewritten: a zero subtracted changes no logit, and a zero
+    // decays to zero under any finite decay (B=7, V=100256, 200 tokens of context: 24.7 -> 20.0 us).
+    unsigned long long pen_mask = ~0ull;
+    auto pen_at = [&](int s) -> bool { return s >= 64 || ((pen_mask >> s) & 1ull) != 0ull; };
     if (rep) {
+        unsigned long long zero_mask = 0ull;
 #pragma unroll 8
         for (int s = 0; s < Kt; s++) {
             float4 v = bulk_load ? row.ld(s) : ldrow4(s * kLanes + tg);
             const float4 q4 = __ldcg(reinterpret_cast<const float4*>(prow) + s * kLanes + tg);
+            if ((__float_as_uint(q4.x) | __float_as_uint(q4.y) | __float_as_uint(q4.z) | __float_as_uint(q4.w)) == 0u && s < 64)
+                zero_mask |= 1ull << s;
             v = scaled4_rep(v, q4, a_scale);
             tmax = fmaxf(fmaxf(fmaxf(tmax, v.x), fmaxf(v.y, v.z)), v.w);
             if (SMEM) row.st(s, v);
         }
+        if (fabsf(p.decay) <= FLT_MAX) pen_mask = ~zero_mask;
     } else {
         int s = 0;
         if (SMEM) {
@@ -494,7 +503,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         l[j] = ldrow4((s + j) * kLanes + tg);
-                        q[j] = __ldcg(q4p + (s + j) * kLanes);
+                        q[j] = pen_at(s + j) ? __ldcg(q4p + (s + j) * kLanes) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
                     scale4x4(l, q);
                 }
@@ -1066,7 +1075,9 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
 #pragma unroll 4
         for (int s = 0; s < Kt; s++) {
             const int i4 = s * kLanes + tg;
-            float4 q4 = __ldcg(reinterpret_cast<const float4*>(prow) + i4);
+            const bool has_pen = pen_at(s);
+            if (!has_pen && i4 != (token >> 2)) continue;
+            const float4 q4 = has_pen ? __ldcg(reinterpret_cast<const float4*>(prow) + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
             float e[4] = {q4.x, q4.y, q4.z, q4.w};
             if (i4 != (token >> 2)) {   // token is -1 outside the owner CTA: no group matches
 #pragma unroll

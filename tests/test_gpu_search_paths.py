@@ -13,21 +13,21 @@ FIELDS_U = ("left", "seqk", "sgtk", "rounds", "idxt", "early_exit")
 FIELDS_F = ("threshold", "comp", "sgtp", "sum_p", "randp", "sum_o", "rand2", "pmin", "pmax")
 
 
-def check_against_oracle(abi, lg, seed, temp, k, p, mode=0, pen=None, rows=4):
+def check_against_oracle(abi, lg, seed, temp, k, p, mode=0, pen=None, rows=4, decay=0.95):
     B, V = lg.shape
     st = abi.setup_rand(seed, B)
     st_cpu = st.cpu().numpy().copy()
     pen_dev = pen.clone().cuda() if pen is not None else None
     abi.set_path(mode)
     try:
-        out, probs, tr = abi.sample(lg.cuda(), st, temp, k, p, penalties=pen_dev, presence=0.1, repetition=0.1, decay=0.95, debug=True)
+        out, probs, tr = abi.sample(lg.cuda(), st, temp, k, p, penalties=pen_dev, presence=0.1, repetition=0.1, decay=decay, debug=True)
     finally:
         abi.set_path(0)
     knd, scale, kk, pp = co.normalise(V, B, 1, temp, k, p, with_penalties=pen is not None)
     for b in sorted({0, B - 1, B // 2, B // 3})[:rows]:
         pen_cpu = pen[b].numpy().copy() if pen is not None else None
         tok, o, _ = co.sample_row(lg[b].numpy(), st_cpu[64 * b:64 * b + 64], knd, scale, kk, pp, penalties=pen_cpu, presence=0.1,
-                                  repetition=0.1, decay=0.95, probs_in=probs[b].cpu().numpy())
+                                  repetition=0.1, decay=decay, probs_in=probs[b].cpu().numpy())
         g = tr[b]
         assert tok == int(out[b]) == g.token, b
         for f in FIELDS_U:
@@ -36,7 +36,8 @@ def check_against_oracle(abi, lg, seed, temp, k, p, mode=0, pen=None, rows=4):
             x, y = np.float32(getattr(o, f)), np.float32(getattr(g, f))
             assert x.view(np.uint32) == y.view(np.uint32), (b, f, x, y)
         if pen is not None:
-            assert np.array_equal(pen_cpu, pen_dev[b].cpu().numpy())
+            assert np.array_equal(pen_cpu, pen_dev[b].cpu().numpy(), equal_nan=True)
+            assert np.array_equal(np.signbit(pen_cpu[pen_cpu == 0]), np.signbit(pen_dev[b].cpu().numpy()[pen_cpu == 0]))
     assert abi.device_status() == 0
     return tr
 
@@ -82,3 +83,17 @@ def test_wide_kept_sets(abi, mode, kind, B, V, temp, k, p):
     if B <= 4 and mode != 1:
         pen = torch.rand(B, V, generator=torch.Generator().manual_seed(2)) * 0.5
         check_against_oracle(abi, make_logits(kind, B, V, 22, torch), 10, temp, k, p, mode, pen=pen)
+
+
+@pytest.mark.parametrize("mode", [0, 2, 3, 4])
+@pytest.mark.parametrize("B,V,density,decay", [(3, 50304, 0.004, 0.95), (130, 4100, 0.0, 0.5), (4, 300000, 0.001, -0.5),
+                                               (150, 32768, 0.02, 0.95), (2, 16384, 0.1, float("inf")), (5, 65536, 1.0, 0.95)])
+def test_zero_penalties_are_neither_copied_nor_rewritten(abi, mode, B, V, density, decay):
+    """Groups whose penalties are all +0 are left alone; -0 becomes +0, a zero times an infinite decay NaN, and the sampled id
+    gets its presence penalty wherever it lies."""
+    g = torch.Generator().manual_seed(3)
+    pen = torch.rand(B, V, generator=g) * (torch.rand(B, V, generator=g) < density)
+    pen[:, 5::97] *= -0.0
+    pen[0] = 0.0
+    tr = check_against_oracle(abi, make_logits("peaked", B, V, 31, torch), 7, 0.8, 50, 0.9, mode, pen=pen, decay=decay)
+    assert all(0 <= t.token < V for t in tr)
