@@ -103,6 +103,21 @@ __device__ __forceinline__ float warp_scan_desc(float v, int lane) {
     return v;
 }
 
+// Sequential prefix over the 32 warp values v of a row, lane w holding that of warp w (sampling.cu:85-92): every lane runs
+// the same chain of additions and keeps the sum that includes its own warp; a thread that needs another warp's prefix
+// takes it by a shuffle.  (A select per warp and value instead was several hundred instructions that run once, bound by
+// their fetch.)
+__device__ __forceinline__ float prefix_seq(float v, int lane, float& total) {
+    float s = __shfl_sync(0xffffffffu, v, 0), mine = s;
+#pragma unroll
+    for (int w = 1; w < kWarps; w++) {
+        s += __shfl_sync(0xffffffffu, v, w);
+        if (lane >= w) mine = s;
+    }
+    total = s;
+    return mine;
+}
+
 // ------------------------------------------------------------- PTX wrappers --------------
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

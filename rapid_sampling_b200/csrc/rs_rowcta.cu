@@ -1042,27 +1042,13 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
     }
     float sum_p, randp;
     {
-        const float4* box4 = reinterpret_cast<const float4*>(box_of(phase));
-        phase ^= 1;
         // sequential prefix over the 32 warp totals (sampling.cu:85-92); this thread needs the prefix before each of
-        // its virtual warps j * WPB + pw, i.e. the running sum after warp w whenever w % WPB == pw - 1
+        // its virtual warps j * WPB + pw
+        const float prefix = prefix_seq(box_of(phase)[lane], lane, sum_p);
+        phase ^= 1;
         float before[LPT];
 #pragma unroll
-        for (int j = 0; j < LPT; j++) before[j] = 0.f;
-        float s0 = 0.f;
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const float4 v = box4[q];
-            const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int w = q * 4 + r;
-                s0 = (w == 0) ? e[r] : s0 + e[r];
-                if ((w % WPB) == pw - 1 && w / WPB < LPT) before[w / WPB] = s0;             // prefix before warp w + 1, same j
-                if (pw == 0 && (w % WPB) == WPB - 1 && w / WPB + 1 < LPT) before[w / WPB + 1] = s0;   // ... next j
-            }
-        }
-        sum_p = s0;
+        for (int j = 0; j < LPT; j++) before[j] = __shfl_sync(FULL, prefix, (j * WPB + pw + 31) & 31);   // (not used by warp 0)
         randp = sum_p * ux;
 #pragma unroll
         for (int j = 0; j < LPT; j++) {
@@ -1088,52 +1074,44 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
     // ---- element pick inside the chosen lane (sampling.cu:725-751) ---------------------------------------------
     __syncthreads();
     const int idxt = *s_idxt;
+    // The lane's elements are played by threads 0, 1, ... of the reference's block, four per stripe: with K stripes only the
+    // first 4 K of them hold one; the warps beyond add zeros and see no transition.
     float oincl[LPT];
     int idn_of[LPT];
 #pragma unroll
     for (int j = 0; j < LPT; j++) {
         const int vt = j * NT + t;   // thread index of the reference block
-        const int idn = idxt * 4 + (vt >> 2) * 4 * kLanes + (vt & 3);
-        float o0 = 0.f;
-        if (idn < V) {
-            const float x = scaled_logit(logit1(idn), rep ? prow[idn] : 0.f, rep, a_scale);
-            o0 = exp2f(x - mx) / denom;
+        oincl[j] = 0.f;
+        idn_of[j] = V;
+        if (j * NT < 4 * K) {
+            const int idn = idxt * 4 + (vt >> 2) * 4 * kLanes + (vt & 3);
+            float o0 = 0.f;
+            if (idn < V) {
+                const float x = scaled_logit(logit1(idn), rep ? prow[idn] : 0.f, rep, a_scale);
+                o0 = exp2f(x - mx) / denom;
+            }
+            const float o = (o0 < thr) ? 0.f : (o0 == thr) ? (o0 * comp) : o0;
+            oincl[j] = warp_scan_desc(o, lane);
+            idn_of[j] = idn;
         }
-        const float o = (o0 < thr) ? 0.f : (o0 == thr) ? (o0 * comp) : o0;
-        oincl[j] = warp_scan_desc(o, lane);
-        idn_of[j] = idn;
         if (lane == 31) s_wtot[vt >> 5] = oincl[j];
     }
     __syncthreads();
     float sum_o, rand2;
     {
-        float opre[LPT];
-#pragma unroll
-        for (int j = 0; j < LPT; j++) opre[j] = 0.f;
-        float s0 = 0.f;
-        const float4* wt4 = reinterpret_cast<const float4*>(s_wtot);
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const float4 v = wt4[q];
-            const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int w = q * 4 + r;
-                s0 = (w == 0) ? e[r] : s0 + e[r];
-                if ((w % WPB) == pw - 1 && w / WPB < LPT) opre[w / WPB] = s0;
-                if (pw == 0 && (w % WPB) == WPB - 1 && w / WPB + 1 < LPT) opre[w / WPB + 1] = s0;
-            }
-        }
-        sum_o = s0;
+        const float prefix = prefix_seq(s_wtot[lane], lane, sum_o);
         rand2 = sum_o * uy;
 #pragma unroll
         for (int j = 0; j < LPT; j++) {
             const int vw = j * WPB + pw;
-            const float cumu_o = (vw > 0) ? oincl[j] + opre[j] : oincl[j];
-            const bool uo = (rand2 <= cumu_o);
-            bool uo_prev = __shfl_up_sync(FULL, uo, 1);
-            if (lane == 0) uo_prev = (vw > 0) ? (rand2 <= opre[j]) : false;
-            if (uo != uo_prev) *s_token = (idn_of[j] < V) ? idn_of[j] : 0;
+            if (j * NT < 4 * K) {
+                const float before = __shfl_sync(FULL, prefix, (vw + 31) & 31);      // (not used by warp 0)
+                const float cumu_o = (vw > 0) ? oincl[j] + before : oincl[j];
+                const bool uo = (rand2 <= cumu_o);
+                bool uo_prev = __shfl_up_sync(FULL, uo, 1);
+                if (lane == 0) uo_prev = (vw > 0) ? (rand2 <= before) : false;
+                if (uo != uo_prev) *s_token = (idn_of[j] < V) ? idn_of[j] : 0;
+            }
         }
     }
     __syncthreads();

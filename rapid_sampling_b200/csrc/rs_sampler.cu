@@ -950,27 +950,11 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     const float actual_p = gtp + (thr * eqk) * comp;
     const float incl = warp_scan_desc(actual_p, lane);
     const uint32_t* lbox = exchange(Packets<1>(), __float_as_uint(__shfl_sync(FULL, incl, 31)), 0u, 0u);   // word 0: warp total
-    float pre_prev = 0.f, sum_p;   // prefix of the warps before mine; total
-    int own_w = -1;                // first warp whose inclusive prefix reaches randp
-    float randp;
-    {
-        // sequential prefix over the warp totals (sampling.cu:85-92)
-        float pre[kWarps];
-        float s0 = 0.f;
-#pragma unroll
-        for (int w = 0; w < kWarps; w++) {
-            const float q = __uint_as_float(bx(lbox, 0, w));
-            s0 = (w == 0) ? q : s0 + q;
-            pre[w] = s0;
-        }
-        sum_p = s0;
-        randp = sum_p * ux;
-#pragma unroll
-        for (int w = kWarps - 1; w >= 0; w--) {
-            if (randp <= pre[w]) own_w = w;
-            if (w == wg - 1) pre_prev = pre[w];
-        }
-    }
+    float sum_p;                   // total
+    const float prefix = prefix_seq(__uint_as_float(bx(lbox, 0, lane)), lane, sum_p);
+    const float pre_prev = __shfl_sync(FULL, prefix, (wg + 31) & 31);      // of the warps before mine (not used by warp 0)
+    const float randp = sum_p * ux;
+    const int own_w = __ffs(__ballot_sync(FULL, randp <= prefix)) - 1;     // first warp whose inclusive prefix reaches randp
     stamp(7);   // totals and lane-pick exchanges done
     const float cumu_p = (wg > 0) ? incl + pre_prev : incl;
     bool u = (randp <= cumu_p);
@@ -994,44 +978,44 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     if (is_owner) {
         __syncthreads();
         const int idxt = *s_idxt;
+        // The lane's elements are played by threads 0, 1, ... of the reference's block, four per stripe: with K stripes only
+        // the first 4 K of them hold one; the warps beyond add zeros and see no transition.
+        const int held = ((V4 + kLanes - 1) >> 10) * 4;
         float oincl[C];
         int idn_of[C];
 #pragma unroll
         for (int it = 0; it < C; it++) {
             const int vt = it * L + t;  // thread index of the reference block
-            const int idn = idxt * 4 + (vt >> 2) * 4 * kLanes + (vt & 3);
-            float o0 = 0.f;
-            if (idn < V) {
-                const float x = scaled_logit(ldrow1(idn), rep ? prow[idn] : 0.f, rep, a_scale);
-                o0 = exp2f(x - mx) / denom;
+            oincl[it] = 0.f;
+            idn_of[it] = V;
+            if (it * L < held) {
+                const int idn = idxt * 4 + (vt >> 2) * 4 * kLanes + (vt & 3);
+                float o0 = 0.f;
+                if (idn < V) {
+                    const float x = scaled_logit(ldrow1(idn), rep ? prow[idn] : 0.f, rep, a_scale);
+                    o0 = exp2f(x - mx) / denom;
+                }
+                const float o = (o0 < thr) ? 0.f : (o0 == thr) ? (o0 * comp) : o0;
+                oincl[it] = warp_scan_desc(o, lane);
+                idn_of[it] = idn;
             }
-            const float o = (o0 < thr) ? 0.f : (o0 == thr) ? (o0 * comp) : o0;
-            oincl[it] = warp_scan_desc(o, lane);
-            idn_of[it] = idn;
             if (lane == 31) s_wtot[vt >> 5] = oincl[it];
         }
         __syncthreads();
-        float opre[C];
-        float s0 = 0.f;
-#pragma unroll
-        for (int it = 0; it < C; it++) opre[it] = 0.f;
-#pragma unroll
-        for (int w = 0; w < kWarps; w++) {
-            s0 = (w == 0) ? s_wtot[0] : s0 + s_wtot[w];
-#pragma unroll
-            for (int it = 0; it < C; it++)
-                if (w == it * WPC + wl - 1) opre[it] = s0;
-        }
-        const float sum_o = s0;
+        float sum_o;
+        const float oprefix = prefix_seq(s_wtot[lane], lane, sum_o);
         const float rand2 = sum_o * uy;
 #pragma unroll
         for (int it = 0; it < C; it++) {
             const int vw = it * WPC + wl;
-            const float cumu_o = (vw > 0) ? oincl[it] + opre[it] : oincl[it];
-            const bool uo = (rand2 <= cumu_o);
-            bool uo_prev = __shfl_up_sync(FULL, uo, 1);
-            if (lane == 0) uo_prev = (vw > 0) ? (rand2 <= opre[it]) : false;
-            if (uo != uo_prev) *s_token = (idn_of[it] < V) ? idn_of[it] : 0;
+            if (it * L < held) {
+                const float before = __shfl_sync(FULL, oprefix, (vw + 31) & 31);      // (not used by warp 0)
+                const float cumu_o = (vw > 0) ? oincl[it] + before : oincl[it];
+                const bool uo = (rand2 <= cumu_o);
+                bool uo_prev = __shfl_up_sync(FULL, uo, 1);
+                if (lane == 0) uo_prev = (vw > 0) ? (rand2 <= before) : false;
+                if (uo != uo_prev) *s_token = (idn_of[it] < V) ? idn_of[it] : 0;
+            }
         }
         __syncthreads();
         token = (*s_fail == 0) ? *s_token : -1;
