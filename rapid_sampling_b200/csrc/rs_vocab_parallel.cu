@@ -147,6 +147,31 @@ __device__ __forceinline__ float vp_cut(uint32_t p_bits, float denom) {
     return p_bits < 0x01000000u ? -INFINITY : log2f(__uint_as_float(p_bits) * denom) - 0.05f;
 }
 
+// Calls body(x - max) for the elements at or above the cut, in chain order.  They are few: noted first, so that the loads run
+// ahead of a loop that holds neither the exponential nor the division (a thread that notes more than kVpNoted sends the
+// whole block through the row once more).
+constexpr int kVpNoted = 8;      // 32 KiB of shared memory
+template <class F>
+__device__ __forceinline__ void vp_select(const VpRow& r, float scale, float mx, float cut, float* s_list, F&& body) {
+    bool noted = cut > -INFINITY;
+    if (noted) {
+        int m = 0;
+        vp_for_each<16>(r, scale, [&](int, float x) {
+            if (x - mx >= cut) {
+                if (m < kVpNoted) s_list[m * kVpThreads + (int)threadIdx.x] = x - mx;
+                m++;
+            }
+        });
+        noted = __syncthreads_or(m > kVpNoted ? 1 : 0) == 0;
+        if (noted)
+            for (int i = 0; i < m; i++) body(s_list[i * kVpThreads + (int)threadIdx.x]);
+    }
+    if (!noted)
+        vp_for_each<8>(r, scale, [&](int, float x) {
+            if (x - mx >= cut) body(x - mx);
+        });
+}
+
 __global__ void __launch_bounds__(kVpThreads) vp_max_kernel(const float* logits, long long row_stride, float* penalties,
                                                             int n, float scale, float* out_max) {
     __shared__ float sh[32];
@@ -206,7 +231,6 @@ __device__ __forceinline__ VpBracket vp_bracket(const float* tallies /* [round][
     return br;
 }
 
-constexpr int kRoundList = 8;      // elements a thread may note in a round (32 KiB)
 // One round: this shard's count and mass at the 15 pivots of the current bracket.  An element below the lowest pivot adds
 // to none of them, and from the second round on nearly all are: they are told by a compare on x alone, and the others are
 // noted first, so that the loads run ahead without 30 sums in registers.  In the first round, whose pivots start at
@@ -216,7 +240,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_round_kernel(const float* logit
                                                               int n, float scale, const float* gmax, const float* gsum,
                                                               const float* tallies, int B, int round, float top_k,
                                                               float top_p, float* out /* [B][15][2] */) {
-    __shared__ float s_list[kRoundList * kVpThreads];
+    __shared__ float s_list[kVpNoted * kVpThreads];
     __shared__ float sh[32 * 32 + 32];
     const int b = blockIdx.x, t = threadIdx.x;
     const VpRow r = vp_row(logits, row_stride, penalties, n, b);
@@ -260,23 +284,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_round_kernel(const float* logit
                 if (j >= shared_pivots && pb >= piv[j]) { v[2 * j] += 1.f; v[2 * j + 1] += p; }
         }
     };
-    bool listed = cut > -INFINITY;
-    if (listed) {
-        int m = 0;
-        vp_for_each<16>(r, scale, [&](int, float x) {
-            if (x - mx >= cut) {
-                if (m < kRoundList) s_list[m * kVpThreads + t] = x - mx;
-                m++;
-            }
-        });
-        listed = __syncthreads_or(m > kRoundList ? 1 : 0) == 0;
-        if (listed)
-            for (int i = 0; i < m; i++) tally(s_list[i * kVpThreads + t]);
-    }
-    if (!listed)
-        vp_for_each<8>(r, scale, [&](int, float x) {
-            if (x - mx >= cut) tally(x - mx);
-        });
+    vp_select(r, scale, mx, cut, s_list, tally);
 #pragma unroll
     for (int j = 0; j < kVpPivots; j++)
         if (j < shared_pivots) { v[2 * j] = cnt_all; v[2 * j + 1] = mass_all; }
@@ -289,6 +297,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_tally_kernel(const float* logit
                                                               int n, float scale, const float* gmax, const float* gsum,
                                                               const float* tallies, int B, int rounds, float top_k,
                                                               float top_p, float* out /* [B][4] */) {
+    __shared__ float s_list[kVpNoted * kVpThreads];
     __shared__ float sh[32 * 3 + 3];
     const int b = blockIdx.x;
     const VpRow r = vp_row(logits, row_stride, penalties, n, b);
@@ -296,14 +305,11 @@ __global__ void __launch_bounds__(kVpThreads) vp_tally_kernel(const float* logit
     const uint32_t thr = vp_bracket(tallies, B, b, rounds, top_k, top_p).left;
     const float cut = vp_cut(thr, denom);
     float v[3] = {0.f, 0.f, 0.f};
-    vp_for_each<16>(r, scale, [&](int, float x) {
-        const float d = x - mx;
-        if (d >= cut) {
-            const float p = exp2f(d) / denom;
-            const uint32_t pb = __float_as_uint(p);
-            if (pb > thr) { v[0] += 1.f; v[1] += p; }
-            if (pb == thr) v[2] += 1.f;
-        }
+    vp_select(r, scale, mx, cut, s_list, [&](float d) {
+        const float p = exp2f(d) / denom;
+        const uint32_t pb = __float_as_uint(p);
+        if (pb > thr) { v[0] += 1.f; v[1] += p; }
+        if (pb == thr) v[2] += 1.f;
     });
     f_block_sums<3>(v, sh);
     if (threadIdx.x == 0) {
@@ -331,6 +337,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_weight_kernel(const float* logi
                                                                const float* tallies, int B, int rounds, float top_k,
                                                                float top_p, int use_p, const float* gtally, int rank,
                                                                int world, float* out /* [B][world] */) {
+    __shared__ float s_list[kVpNoted * kVpThreads];
     __shared__ float sh[32];
     const int b = blockIdx.x;
     const VpRow r = vp_row(logits, row_stride, penalties, n, b);
@@ -339,9 +346,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_weight_kernel(const float* logi
     const float comp = vp_comp(gtally + b * 4, thr, top_k, top_p, use_p != 0);
     const float cut = vp_cut(__float_as_uint(thr), denom);       // below it the weight is zero
     float acc = 0.f;
-    vp_for_each<16>(r, scale, [&](int, float x) {
-        if (x - mx >= cut) acc += vp_weight_of(exp2f(x - mx) / denom, thr, comp);
-    });
+    vp_select(r, scale, mx, cut, s_list, [&](float d) { acc += vp_weight_of(exp2f(d) / denom, thr, comp); });
     const float s = vp_block_sum(acc, sh);
     if (threadIdx.x == 0) out[(long long)b * world + rank] = s;
 }
@@ -405,8 +410,8 @@ __global__ void __launch_bounds__(kVpThreads) vp_pick_kernel(const float* logits
     }
     // The weight before a column is a chain over (chunk of 1024 columns, warp of the chunk): the warps' scans are summed in
     // that order.  All warps first compute their totals for up to kPickChunks chunks at once (most are zero and need no
-    // more than a compare per column); warp 0 then walks the totals that are not zero -- adding a zero changes nothing
-    // -- and looks inside a warp's columns only where the target is reached (B=32, 131072 columns: 146 -> 94 us).
+    // more than a compare per column); warp 0 then adds up whole chunks -- adding a zero changes nothing -- and looks
+    // inside a warp's columns only where the target is reached (B=32, 131072 columns: 146 -> 80 us).
     const float cut = vp_cut(__float_as_uint(thr), denom);
     int last = -1;                                   // last column of positive weight that this lane has seen
     for (int base = 0; base < n; base += kPickChunks * kVpThreads) {
@@ -436,7 +441,16 @@ __global__ void __launch_bounds__(kVpThreads) vp_pick_kernel(const float* logits
             int found = 0x7fffffff;
             for (int c = 0; c < chunks && found == 0x7fffffff; c++) {
                 const float mine = s_tot[c * 32 + lane];
-                for (unsigned nz = __ballot_sync(0xffffffffu, mine != 0.f); nz; nz &= nz - 1u) {
+                const unsigned any = __ballot_sync(0xffffffffu, mine != 0.f);
+                if (any == 0u) continue;
+                float end = run;
+#pragma unroll
+                for (int k = 0; k < 32; k++) end += __shfl_sync(0xffffffffu, mine, k);
+                if (!(target <= end)) {              // not in this chunk
+                    run = end;
+                    continue;
+                }
+                for (unsigned nz = any; nz; nz &= nz - 1u) {
                     const int k = __ffs(nz) - 1;
                     const float pre = run;
                     run = run + __shfl_sync(0xffffffffu, mine, k);
