@@ -29,7 +29,7 @@ struct Params {
     const struct RowArgs* rows;   // per-row parameters (ROWP kernels only), else null
     float* out_prob;         // optional B: probability of the sampled id (ROWP kernels only)
     float* out_kept;         // optional B: kept probability mass the id was drawn from (ROWP kernels only)
-    int quick;               // 1: try the one-warp search on integer masses first; 0 (test instrumentation): exact search only
+    int quick;               // 1: try the search on integer masses first; 0 (test instrumentation): exact search only
 };
 
 // Normalised parameters of one row, made on the device from the caller's per-row tensors.

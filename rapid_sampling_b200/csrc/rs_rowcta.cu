@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
     uint32_t beta_p = 0u;
     uint32_t list_total = (uint32_t)V, list_left = 0u;
     bool whole = false;
-    int quick = 0;           // outcome of the one-warp search on integer masses: 0 not settled that way, 1 settled, 2 list too short
+    int quick = 0;           // outcome of the search on integer masses: 0 not settled that way, 1 settled, 2 list too short
     auto lane_eval = [&](const float (&f)[4], uint32_t lo, uint32_t hi, uint32_t cnt_lo, float (&m)[NV], uint32_t (&c)[4],
                          uint32_t& mn, uint32_t& mxv) {
         c[0] = c[1] = c[2] = c[3] = 0u;

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     volatile uint32_t* s_res = reinterpret_cast<volatile uint32_t*>(smem + kMiscOff + 192);   // ten combined words of an exchange
     volatile int* s_fail = reinterpret_cast<volatile int*>(smem + kMiscOff + 32);             // set when a bounded wait of this CTA gave up
     uint64_t* qbar = reinterpret_cast<uint64_t*>(smem + kMiscOff + 40);                       // counts the bytes of the unordered candidate list
-    volatile uint32_t* s_quick = reinterpret_cast<volatile uint32_t*>(smem + kMiscOff + 48);  // outcome of the one-warp search: left, right, rounds, verdict
+    volatile uint32_t* s_quick = reinterpret_cast<volatile uint32_t*>(smem + kMiscOff + 48);  // outcome of the search on integer masses: left, right, rounds, verdict
     uint2* qlist = reinterpret_cast<uint2*>(smem + kQuickOff);
     uint32_t* qsum = reinterpret_cast<uint32_t*>(smem + kQsumOff);
     if (t < 64) qsum[t] = 0u;      // (ordered by the barrier that follows the mbarriers' set-up)
@@ -668,7 +668,8 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     //    its carried state keeps the loop going -- all it uses these values for.  Otherwise: not valid.
     //  * bounds: the smallest and largest element inside the zone move its ends up to them without an evaluation.
     // `lane_eval(f, keep, lo, hi, cnt_keep, ...)` returns this lane's ordered masses and counts at four points, and the
-    // bounds of its elements in [lo, hi); elements below `keep` (there are cnt_keep from it on) will not be asked for again.
+    // bounds of its elements in [lo, hi), of which the row has `inside` at most (0 and 2^31 - 1: not tracked, there are too many);
+    // elements below `keep` (there are cnt_keep from it on) will not be asked for again.
     auto run_search = [&](auto&& lane_eval, const bool clamp, const uint32_t beta_p, const bool sure_cnt) -> bool {
         const uint32_t ustar = clamp ? beta_p + 1u : 0u;
         left = __float_as_uint(pmin);
@@ -726,7 +727,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
                 const float f[4] = {__uint_as_float(u[0]), __uint_as_float(u[1]), __uint_as_float(u[2]), __uint_as_float(u[3])};
                 float m[4], mass[4];
                 uint32_t cnt[4], c01, c23, mn, mxv, vmin, vmax;
-                lane_eval(f, za > 0u ? za - 1u : 0u, za, zb, cnt_a, m, c01, c23, mn, mxv);
+                lane_eval(f, za > 0u ? za - 1u : 0u, za, zb, cnt_a, cnt_a - cnt_b, m, c01, c23, mn, mxv);
                 totals(m, c01, c23, mn, mxv, cnt, mass, vmin, vmax);
                 const uint32_t za_old = za, w_old = zb - za;
                 // the highest point that exceeds, the lowest that passes
@@ -768,6 +769,90 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             }
         }
         return !clamp || left > beta_p;
+    };
+
+    // Short rows (V <= 4096, where the bound admits every element to the list) are searched at the reference's own pivots, three a
+    // round: a lane holds an element or two, an evaluation is all exchange, and the placing of the points costs more
+    // than the rounds it saves (B=19, V=1668, top_p 0.3: 18.4 us against 21.2).
+    //  * frozen: once every element strictly inside (left, right) has one and the same value v, the remaining rounds need
+    //    no data: a pivot equal to `left` selects the set of `left`, a pivot in (left, v] the set {p >= v}, a pivot above v
+    //    the set of `right`; they are replayed arithmetically.  A closed bracket carries the totals at its upper end.
+    uint32_t conv_cnt = 0, conv_left_cnt = 0;   // counts at `right` / `left` and ordered mass at `right` on return
+    float conv_mass = 0.f;
+    bool carried = false;
+    auto replay_search = [&](auto&& lane_eval, const bool clamp, const uint32_t beta_p, const bool sure_cnt,
+                          const uint32_t n_above) -> bool {
+        const uint32_t ustar = clamp ? beta_p + 1u : 0u;
+        left = __float_as_uint(pmin);
+        right = __float_as_uint(pmax) + 1u;
+        rounds = 0;
+        uint32_t cnt_x = (uint32_t)V, cnt_r = 0u;   // counts at left / at right
+        float mass_x = 1.0f, mass_r = 0.f;
+        bool frozen = false, valid = true;
+        uint32_t v_bits = 0, cnt_v = 0;
+        float mass_v = 0.f;
+        while (rounds < 64u) {
+            const bool go = use_cnt ? (cnt_x > top_k || mass_x > top_p) : (mass_x > top_p);
+            if (!(go && left < right - 1u)) break;
+            rounds++;
+            const uint32_t pz = (left + right) >> 1, py = (left + pz) >> 1, pw = (pz + right) >> 1;
+            const uint32_t pv[3] = {py, pz, pw};
+            uint32_t cnt[4];
+            float mass[4];
+            if (clamp && sure_cnt && pw <= beta_p) {
+                // All three pivots lie at or below the bound, and more than top_k elements are known to lie
+                // strictly above it: every test fails, the lower end moves to the last pivot, no data is needed.
+                left = pw;
+                cnt_x = n_above;
+                mass_x = 0.f;
+                continue;
+            }
+            if (!frozen) {
+                n_eval++;
+                const float f[4] = {__uint_as_float(max(py, ustar)), __uint_as_float(max(pz, ustar)),
+                                    __uint_as_float(max(pw, ustar)), __uint_as_float(max(left + 1u, ustar))};
+                float m[4];
+                uint32_t c01, c23, mn, mxv, vmin, vmax;
+                lane_eval(f, left, right, cnt_x, m, c01, c23, mn, mxv);
+                totals(m, c01, c23, mn, mxv, cnt, mass, vmin, vmax);
+                if (clamp && left >= beta_p && vmin >= vmax) {   // one distinct value inside (none: vmin > vmax)
+                    frozen = true;
+                    v_bits = (vmin == vmax) ? vmin : left;
+                    cnt_v = cnt[3];      // the set {p >= left + 1} is {p >= v}
+                    mass_v = mass[3];
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const bool at_left = (pv[i] == left), le_v = (pv[i] <= v_bits);
+                    cnt[i] = at_left ? cnt_x : le_v ? cnt_v : cnt_r;
+                    mass[i] = at_left ? mass_x : le_v ? mass_v : mass_r;
+                }
+            }
+            // the three tests and the bracket update, written with selects: this is the critical path of every round
+            bool ok[3], bad = false;
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const bool below = clamp && pv[i] <= beta_p;
+                const bool exceeds = (use_cnt && cnt[i] > top_k) || mass[i] > top_p;
+                const bool pass = (!use_cnt || cnt[i] < top_k) && mass[i] < top_p;
+                ok[i] = !below && pass;
+                bad = bad || (below && !exceeds);
+            }
+            if (bad) { valid = false; break; }
+            const bool s0 = ok[0], s1 = !s0 && ok[1], s2 = !s0 && !s1 && ok[2];   // none: the bracket's upper part
+            const uint32_t nl = s0 ? left : s1 ? py : s2 ? pz : pw;
+            const uint32_t nr = s0 ? py : s1 ? pz : s2 ? pw : right;
+            const uint32_t ncx = s0 ? cnt_x : s1 ? cnt[0] : s2 ? cnt[1] : cnt[2];
+            const float nmx = s0 ? mass_x : s1 ? mass[0] : s2 ? mass[1] : mass[2];
+            const uint32_t ncr = s0 ? cnt[0] : s1 ? cnt[1] : s2 ? cnt[2] : cnt_r;
+            const float nmr = s0 ? mass[0] : s1 ? mass[1] : s2 ? mass[2] : mass_r;
+            left = nl; right = nr; cnt_x = ncx; mass_x = nmx; cnt_r = ncr; mass_r = nmr;
+        }
+        conv_cnt = cnt_r;
+        conv_mass = mass_r;
+        conv_left_cnt = cnt_x;
+        return valid && (!clamp || left > beta_p);
     };
 
     float gtp = 0.f;         // this lane's mass above the threshold, its ties with it, its count above
@@ -858,20 +943,25 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             list_total = (uint32_t)V;
             list_left = left;
         }
-        auto list_eval = [&](const float (&f)[4], uint32_t keep, uint32_t lo, uint32_t hi, uint32_t cnt_keep, float (&m)[4], uint32_t& c01,
-                             uint32_t& c23, uint32_t& mn, uint32_t& mxv) {
+        auto list_eval = [&](const float (&f)[4], uint32_t keep, uint32_t lo, uint32_t hi, uint32_t cnt_keep, uint32_t inside, float (&m)[4],
+                             uint32_t& c01, uint32_t& c23, uint32_t& mn, uint32_t& mxv) {
             if (keep != list_left && cnt_keep * 2u <= list_total) {
                 // half of the list will not be asked for again: dropped in place, order preserved
                 const float kf = __uint_as_float(keep);
                 int q = 0;
-                for (int i = 0; i < n; i += 4) {
-                    const float4 v = lbase[(i >> 2) * lstride];
-                    const float e[4] = {v.x, v.y, v.z, v.w};
+                for (int i = 0; i < n; i += 8) {
+                    float4 v[2];      // loaded together; a place is written only after it has been read
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if (e[j] >= kf) {
-                            reinterpret_cast<float*>(lbase + (q >> 2) * lstride)[q & 3] = e[j];
-                            q++;
+                    for (int h = 0; h < 2; h++) v[h] = (i + 4 * h < n) ? lbase[((i >> 2) + h) * lstride] : make_float4(-1.f, -1.f, -1.f, -1.f);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const float e[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            if (e[j] >= kf) {
+                                reinterpret_cast<float*>(lbase + (q >> 2) * lstride)[q & 3] = e[j];
+                                q++;
+                            }
                         }
                     }
                 }
@@ -880,31 +970,81 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
                 list_total = cnt_keep;
                 list_left = keep;
             }
-            mn = 0xffffffffu;
-            mxv = 0u;
-            m[0] = m[1] = m[2] = m[3] = 0.f;
+            float m0 = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
             c01 = c23 = 0u;
-#pragma unroll 2
-            for (int i = 0; i < n; i += 4) {
-                const float4 v = lbase[(i >> 2) * lstride];
-                const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float q = e[j];
-                    const uint32_t qb = __float_as_uint(q);
-                    const bool in = qb >= lo && qb < hi;          // (the padding's bits are above any hi)
+            // Few warps share an SM in the on-chip variant: a branch per element and point would wait out its latency each time
+            // (B=2, V=285288, flat, bf16: 108 us with branches, 66 us with selects; adding zero changes no sum of terms >= 0).
+            // The streaming variant fills the SM and is bound by issue, where skipped instructions count (B=100, V=71344,
+            // flat: 101 us with selects and bounds throughout, 90 us).
+            auto add = [&](const float q) {
+                if constexpr (SMEM) {
                     c01 += (q >= f[0] ? 1u : 0u) + (q >= f[1] ? 0x10000u : 0u);
                     c23 += (q >= f[2] ? 1u : 0u) + (q >= f[3] ? 0x10000u : 0u);
-                    m[0] += q >= f[0] ? q : 0.f;                  // (adding zero changes no sum of terms >= 0)
-                    m[1] += q >= f[1] ? q : 0.f;
-                    m[2] += q >= f[2] ? q : 0.f;
-                    m[3] += q >= f[3] ? q : 0.f;
-                    mn = min(mn, in ? qb : 0xffffffffu);
-                    mxv = max(mxv, in ? qb : 0u);
+                    m0 += q >= f[0] ? q : 0.f;
+                    m1 += q >= f[1] ? q : 0.f;
+                    m2 += q >= f[2] ? q : 0.f;
+                    m3 += q >= f[3] ? q : 0.f;
+                    return;
+                }
+                if (q >= f[0]) { c01 += 1u; m0 += q; }
+                if (q >= f[1]) { c01 += 0x10000u; m1 += q; }
+                if (q >= f[2]) { c23 += 1u; m2 += q; }
+                if (q >= f[3]) { c23 += 0x10000u; m3 += q; }
+            };
+            if (SMEM || inside <= 256u) {
+                mn = 0xffffffffu;
+                mxv = 0u;
+#pragma unroll 2
+                for (int i = 0; i < n; i += 4) {
+                    const float4 v = lbase[(i >> 2) * lstride];
+                    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        add(e[j]);
+                        const uint32_t qb = __float_as_uint(e[j]);      // (the padding's bits are above any hi)
+                        const bool in = qb >= lo && qb < hi;
+                        mn = min(mn, in ? qb : 0xffffffffu);
+                        mxv = max(mxv, in ? qb : 0u);
+                    }
+                }
+            } else {
+                mn = 0u;
+                mxv = 0x7fffffffu;      // not tracked
+#pragma unroll 4
+                for (int i = 0; i < n; i += 4) {
+                    const float4 v = lbase[(i >> 2) * lstride];
+                    add(v.x); add(v.y); add(v.z); add(v.w);
                 }
             }
+            m[0] = m0; m[1] = m1; m[2] = m2; m[3] = m3;
         };
-        if (quick != 1 && !run_search(list_eval, !whole, beta_p, !whole && use_cnt && nstrict > top_k) && !whole) continue;
+        if (quick != 1) {
+            bool ok;
+            if (!whole && V <= 4096) {
+                const int m_own = n;
+                auto cand_eval = [&](const float (&f)[4], uint32_t lo, uint32_t hi, uint32_t, float (&m)[4], uint32_t& c01,
+                                     uint32_t& c23, uint32_t& mn, uint32_t& mxv) {
+                    m[0] = m[1] = m[2] = m[3] = 0.f;
+                    c01 = c23 = 0u;
+                    mn = 0xffffffffu;
+                    mxv = 0u;
+                    for (int i = 0; i < m_own; i++) {
+                        const float q = cand_at(i);
+                        const uint32_t qb = __float_as_uint(q);
+                        if (q >= f[0]) { c01 += 1u; m[0] += q; }
+                        if (q >= f[1]) { c01 += 0x10000u; m[1] += q; }
+                        if (q >= f[2]) { c23 += 1u; m[2] += q; }
+                        if (q >= f[3]) { c23 += 0x10000u; m[3] += q; }
+                        if (qb > lo && qb < hi) { mn = min(mn, qb); mxv = max(mxv, qb); }
+                    }
+                };
+                ok = replay_search(cand_eval, true, beta_p, use_cnt && nstrict > top_k, nstrict);
+                carried = ok;
+            } else {
+                ok = run_search(list_eval, !whole, beta_p, !whole && use_cnt && nstrict > top_k);
+            }
+            if (!ok && !whole) continue;
+        }
         // recount at the threshold (sampling.cu:657-680)
         const float thr = __uint_as_float(left);
         for (int i = 0; i < n; i += 4) {
@@ -928,7 +1068,13 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     // same tree value as the butterfly, and the warp values are then added in warp order.
     float sgtp;
     uint32_t seqk, sgtk;
-    {
+    if (carried && !early_exit) {
+        // The bracket closed (right == left + 1): the set at `right` is exactly {p > threshold}, and its count
+        // and ordered mass were carried along by the search; the ties are the rest of the set at `left`.
+        sgtp = conv_mass;
+        sgtk = conv_cnt;
+        seqk = conv_left_cnt - conv_cnt;
+    } else {
         const float m[4] = {gtp, 0.f, 0.f, 0.f};
         uint32_t cnt[4], d0, d1;
         float mass[4];
@@ -1437,7 +1583,11 @@ static int sample_rows_impl(const void* logits, int dtype, int64_t B, int64_t T,
     {   // large batches: one CTA per row, as for per-call parameters
         const int mode = g_path_override.load();
         const bool eligible = workspace_bytes - rab >= ws_bytes(B, V);
-        const bool wanted = (mode == 4 || mode == 5) || ((mode == 0 || mode == 6) && g_cluster_override.load() == 0 && !pl.smem && B >= kRowCtaMinBatch);
+        // ... if the rows are short: among rows that bring their own settings some have no top_k and search much of their row,
+        // and the call lasts as long as they do (a mix of settings, one CTA per row against streaming: B=133 V=106860 bf16
+        // 200.7 / 90.2 us, B=256 V=65536 with penalties 279.0 / 123.7, B=300 V=16384 bf16 95.7 / 64.9)
+        const bool wanted = (mode == 4 || mode == 5) ||
+                            ((mode == 0 || mode == 6) && g_cluster_override.load() == 0 && !pl.smem && B >= kRowCtaMinBatch && V <= 8192);
         if (eligible && wanted) {
             pl.rowcta = true;
             pl.ws = ws_bytes(B, V);
