@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     // pivot on its far side: points below `za` are known to exceed top_k or top_p, points from `zb` on pass, points in
     // [e0, e1] do neither.  Pivots inside the unknown zone [za, zb) are settled by evaluating four points of our own
     // choice, placed by interpolation on mass and count, which close in on the boundary much faster than the pivots'
-    // quartering: about 6 evaluations instead of 12 to 15 (B=4, V=131072, flat: 49.6 -> 45.0 us a call).
+    // quartering: about 6 evaluations instead of 12 to 15 (B=4, V=131072, flat: 49.6 -> 45.1 us a call).
     //  * clamp (candidate list only): every probability above beta_p is on the list, so a pivot above beta_p
     //    sees exactly the elements the reference sees.  A pivot u <= beta_p is not evaluated; instead the set
     //    {p > beta_p} is (pivot u*, the next float after beta_p): if it already holds more than top_k elements
@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             float m0 = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
             c01 = c23 = 0u;
             // Few warps share an SM in the on-chip variant: a branch per element and point would wait out its latency each time
-            // (B=2, V=285288, flat, bf16: 108 us with branches, 66 us with selects; adding zero changes no sum of terms >= 0).
+            // (B=2, V=285288, flat, bf16: 108 us with branches, 69 us with selects; adding zero changes no sum of terms >= 0).
             // The streaming variant fills the SM and is bound by issue, where skipped instructions count (B=100, V=71344,
             // flat: 101 us with selects and bounds throughout, 90 us).
             auto add = [&](const float q) {
