@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         left = __float_as_uint(pmin);
         right = __float_as_uint(pmax) + 1u;
         rounds = 0;
-        uint32_t za = max(left, ustar) + ((clamp && sure_cnt) ? 1u : 0u), zb = right;
+        uint32_t za = max(left, ustar), zb = right;
         uint32_t e0 = 1u, e1 = 0u;                        // none yet
         uint32_t cnt_a = (uint32_t)V, cnt_b = 0u;         // of the sets at za - 1 and zb (estimates until evaluated)
         float mass_a = 1.0f, mass_b = 0.f;
@@ -688,6 +688,9 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             const uint32_t pz = (left + right) >> 1, py = (left + pz) >> 1, pw = (pz + right) >> 1;
             // 2 exceeds, 1 neither, 0 passes, -1 unknown
             auto known = [&](uint32_t u) -> int {
+                // More than top_k elements have e > beta_e: their quotients are >= beta_p, so a pivot up to beta_p exceeds.
+                // beta_p + 1 need not: many e above beta_e may share the quotient beta_p.  It is evaluated like any other.
+                if (clamp && sure_cnt && u <= beta_p) return 2;
                 u = max(u, ustar);
                 return u < za ? 2 : u >= zb ? 0 : (u >= e0 && u <= e1) ? 1 : -1;
             };

@@ -24,7 +24,7 @@ def check_against_oracle(abi, lg, seed, temp, k, p, mode=0, pen=None, rows=4, de
     finally:
         abi.set_path(0)
     knd, scale, kk, pp = co.normalise(V, B, 1, temp, k, p, with_penalties=pen is not None)
-    for b in sorted({0, B - 1, B // 2, B // 3})[:rows]:
+    for b in (range(B) if rows >= B else sorted({0, B - 1, B // 2, B // 3})[:rows]):
         pen_cpu = pen[b].numpy().copy() if pen is not None else None
         tok, o, _ = co.sample_row(lg[b].numpy(), st_cpu[64 * b:64 * b + 64], knd, scale, kk, pp, penalties=pen_cpu, presence=0.1,
                                   repetition=0.1, decay=decay, probs_in=probs[b].cpu().numpy())
@@ -97,3 +97,24 @@ def test_zero_penalties_are_neither_copied_nor_rewritten(abi, mode, B, V, densit
     pen[0] = 0.0
     tr = check_against_oracle(abi, make_logits("peaked", B, V, 31, torch), 7, 0.8, 50, 0.9, mode, pen=pen, decay=decay)
     assert all(0 <= t.token < V for t in tr)
+
+
+@pytest.mark.parametrize("mode", [0, 2, 3, 4, 6])     # the planner's choice, streaming, on-chip, one CTA per row, exact search only
+@pytest.mark.parametrize("V,low,near,top", [(6144, 6024, 100, 20), (8192, 7282, 900, 10), (12000, 11800, 180, 20), (30000, 29300, 690, 10)])
+def test_elements_above_the_bound_whose_quotients_tie_with_it(abi, mode, V, low, near, top):
+    """Rows of a few large logits, some that lie one to three floats above the rest, and the rest: the bound of the candidate
+    list falls on the rest, more than top_k elements lie above it, and after the division by the denominator many of those tie
+    with it, so that the cutoff is the bound's own probability."""
+    B, k = 48, 50
+    rng = np.random.default_rng(V + near)
+    lg = np.empty((B, V), np.float32)
+    for b in range(B):
+        x = np.float32(rng.uniform(-1.0, 1.0))
+        rest = np.full(V, x, np.float32)
+        up = x
+        for _ in range(1 + b % 3):
+            up = np.nextafter(up, np.float32(4))
+            rest[low:low + near][rng.random(near) < (1.0 if up == np.nextafter(x, np.float32(4)) else 0.5)] = up
+        rest[low + near:] = np.float32(x + rng.uniform(0.5, 1.0))
+        lg[b] = rng.permutation(rest)
+    check_against_oracle(abi, torch.from_numpy(lg), 3, 1.0, k, 1.0, mode, rows=B)
