@@ -412,13 +412,15 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     uint32_t ncand, nstrict;
     const uint32_t* p2box = nullptr;   // the mailbox of the last collection: word 4 = candidates of each virtual warp
     // How far to lower the bound is read off a histogram of a quarter of the elements below it, in eighths of an octave
-    // (calls whose cutoff a large top_p decides; the others' lists are almost never too thin).  It uses the words that
-    // the search's sample sums need later, and leaves them cleared.
+    // (calls whose cutoff a large top_p decides; the others' lists are almost never too thin; and rows of which every lane
+    // holds a batch of four groups, one of which is the sample).  It uses the words that the search's sample sums need
+    // later, and leaves them cleared.
     const bool want_hist = try_cand && a_top_k >= V && a_top_p > 0.5f && V >= 16384;
-    const float sampled = (float)V4 / (float)(max(V4 >> 12, 1) << 10);      // elements that a sampled one stands for
     const uint32_t beta_bits = __float_as_uint(beta_e);
+    float tail = 0.f;      // mass of the sampled elements below the histogram
     auto sample1 = [&](float e) {
-        const uint32_t bin = (beta_bits - __float_as_uint(e)) >> 20;      // (an element above the bound: a huge number)
+        const uint32_t bits = __float_as_uint(e), bin = (beta_bits - bits) >> 20;      // (an element above the bound: a huge number)
+        tail += (bits < beta_bits && bin >= 64u) ? e : 0.f;
         if (bin < 64u) atomicAdd(qsum + bin, 1u);
     };
     auto append = [&](const float4 v) {
@@ -561,47 +563,56 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         emax = warp_max(__uint_as_float(bx(box, 2, lane)));
         cmass = judge(box);
     }
-    for (int attempt = 0; attempt < 2 && cand_ok && !enough && beta_e > 0.f; attempt++) {
+    bool last_attempt = false;
+    for (int attempt = 0; attempt < 2 && cand_ok && !enough && !last_attempt && beta_e > 0.f; attempt++) {
         float lowered = beta_e * 0.0625f;
         if (attempt == 0 && want_hist) {
-            // The CTAs' histograms as estimates of mass and count between the bound and 1, 2, 3, 5 and 8 octaves below it,
-            // added up over the cluster: the first of these levels that makes up the missing mass, with a margin for the
-            // sampling.  A level that would not fit the lists, or none: the whole row is searched.
-            uint32_t wa = 0u, wb = 0u, wc = 0u;
+            // The CTAs' histograms, two bins together, added up over the cluster: lane l estimates the count between the bound
+            // and l + 1 quarter octaves below it, and the mass that such a list would leave out.  (That mass and not the
+            // list's own: its elements are the smaller and more numerous ones, so that the sample tells it more sharply.)
+            // Taken is the first level that leaves out no more than the cutoff allows, with 2 % for the place inside a bin
+            // and four standard deviations of the sample to spare; if its list would not fit, the deepest that fits, as long
+            // as it needs nothing to spare.  Otherwise the whole row is searched: a list that turns out too thin or too long
+            // costs its pass over the row.  (Estimating the list's own mass at 1, 2, 3, 5 and 8 octaves, with 5 % to spare and
+            // half of the buffer as its longest list, sent rows with a wide head to the whole-row search: B=32, V=1048576, 1 % of
+            // the ids raised by 8, top_p 0.95: 439 -> 192 us a call; lowering 16-fold without a look: 293.)
+            // elements that a sampled one stands for: one group of every whole four of a lane is sampled, and V4 & 1023 lanes hold
+            // one group more than the others
+            const float sampled = (float)V4 / (float)max((V4 & 1023) * (((V4 >> 10) + 1) >> 2) + (kLanes - (V4 & 1023)) * (V4 >> 12), 1);
+            uint32_t wa = 0u, wb = 0u;
             __syncthreads();
-            if (wl == 0) {         // lane l: bins l and l + 32; one octave is eight bins
-                const float n0 = sampled * (float)qsum[lane], n1 = sampled * (float)qsum[lane + 32];
-                const float m0 = n0 * beta_e * exp2f(-0.125f * (float)(lane + 1)), m1 = n1 * beta_e * exp2f(-0.125f * (float)(lane + 33));
-                // running sums over the bins, read off where the levels end
-                const float cm = warp_scan_desc(m0, lane), cn = warp_scan_desc(n0, lane);
-                const float dm = __shfl_sync(FULL, cm, 31) + warp_scan_desc(m1, lane), dn = __shfl_sync(FULL, cn, 31) + warp_scan_desc(n1, lane);
-                auto at = [&](float v, int l) { return __float_as_uint(__shfl_sync(FULL, v, l)); };
-                const uint32_t a0 = at(cm, 7), a1 = at(cm, 15), a2 = at(cm, 23), a3 = at(dm, 7), a4 = at(dm, 31);
-                const uint32_t b0 = at(cn, 7), b1 = at(cn, 15), b2 = at(cn, 23), b3 = at(dn, 7), b4 = at(dn, 31);
-                wa = pick4(a0, a1, a2, a3);
-                wb = pick4(a4, b0, b1, b2);
-                wc = pick4(b3, b4, 0u, 0u);
+            if (wl < 2) {          // warp w: levels 16 w to 16 w + 15, two to a word, four words from lanes 0, 8, 16, 24 each
+                const uint32_t n = (lane < 16) ? min(qsum[(wl * 16 + lane) * 2] + qsum[(wl * 16 + lane) * 2 + 1], 0xffffu) : 0u;
+                const uint32_t w = n | (__shfl_down_sync(FULL, n, 1) << 16);      // (lane 2 k: word k)
+                wa = __shfl_sync(FULL, w, 2 * xk);
+                wb = __shfl_sync(FULL, w, 2 * xk + 8);
             }
-            const uint32_t* box = exchange(Packets<3>(), wa, wb, wc);
-            float word = 0.f;                      // lane k: word k, added up over the CTAs (their first warps)
-            if (lane < 10) {
+            const uint32_t* box = exchange(Packets<3>(), wa, wb, __float_as_uint(warp_tree_sum(tail)));
+            uint32_t n = 0u;
 #pragma unroll
-                for (int c = 0; c < C; c++) word += __uint_as_float(bx(box, lane, c * WPC));
-            }
-            const float need = fmaxf(a_top_p * 1.002f - cmass, 0.f) * denom * 1.05f;
-            const float room = 0.5f * (float)(cap * kLanes) - (float)ncand;
-            lowered = -1.f;
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                const float mk = __shfl_sync(FULL, word, k), ck = __shfl_sync(FULL, word, 5 + k);
-                const float level = k == 0 ? 0.5f : k == 1 ? 0.25f : k == 2 ? 0.125f : k == 3 ? 0.03125f : 0.00390625f;
-                if (lowered < 0.f && mk >= need) lowered = (ck <= room) ? beta_e * level : 0.f;
-            }
-            if (lowered <= 0.f && V > cap * kLanes) {
+            for (int c = 0; c < C; c++) n += (bx(box, (lane >> 1) & 7, c * WPC + (lane >> 4)) >> ((lane & 1) * 16)) & 0xffffu;
+            const uint32_t mid = ((uint32_t)lane << 21) + (1u << 20), low = (uint32_t)(lane + 1) << 21;
+            const float em = __uint_as_float(beta_bits > mid ? beta_bits - mid : 0u), nf = (float)n;
+            const float below = warp_tree_sum(__uint_as_float(bx(box, 8, lane)));
+            float m1 = warp_scan_desc(nf * em, lane), m2 = warp_scan_desc(nf * em * em, lane);
+            m1 = sampled * (__shfl_sync(FULL, m1, 31) - m1 + below);
+            // (each of the tail's elements is smaller than beta_e / 256; one element at the level itself may have gone unsampled)
+            m2 = __shfl_sync(FULL, m2, 31) - m2 + below * beta_e * 0.00390625f + em * em;
+            m2 = 4.f * sqrtf(sampled * fmaxf(sampled - 1.f, 0.f) * fmaxf(m2, 0.f));
+            // the fullest lane of a list of so many elements: the mean and 4.2 standard deviations (1024 lanes: about one list
+            // in 25 has a fuller one)
+            const float mean = ((float)ncand + sampled * warp_scan_desc(nf, lane)) * (1.f / kLanes), all = (float)V * (1.f / kLanes);
+            const bool fits = all <= (float)cap || mean + 4.2f * sqrtf(mean * fmaxf(1.f - mean / all, 0.f)) <= (float)cap;
+            const float spare = (1.f - a_top_p * 1.0015f) * denom;
+            const unsigned reach = __ballot_sync(FULL, m1 * 1.02f + m2 <= spare), likely = __ballot_sync(FULL, m1 <= spare);
+            const unsigned fit = __ballot_sync(FULL, fits);
+            const int level = min(reach ? __ffs(reach) - 1 : 31, 31 - __clz(fit));
+            if (level < 0 || ((likely >> level) & 1u) == 0u) {
                 cand_ok = false;
                 break;
             }
-            lowered = fmaxf(lowered, 0.f);
+            lowered = __shfl_sync(FULL, __uint_as_float(beta_bits > low ? beta_bits - low : 0u), level);
+            last_attempt = level < 31;      // (a list that turns out too thin all the same cannot grow much)
         }
         // a flat row: the lowered bound would already admit every element.  Either the whole row fits the candidate
         // buffer (no bound at all), or there is no point in trying.
@@ -633,6 +644,8 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         csum = warp_tree_sum(csum);
         cmass = judge(exchange(Packets<2>(), pick4(0u, 0u, 0u, overflow), pick4(wnc, wns, __float_as_uint(csum), 0u), 0u));
     }
+    // neither more than top_k elements nor (clear of the roundings) the mass: no cutoff lies above the bound
+    if (!enough && cmass < a_top_p * 0.99999f) cand_ok = false;
     if (want_hist && wl == 0) qsum[lane] = qsum[lane + 32] = 0u;
     // division is monotone, so the row's min/max probability are the quotients of min/max e
     const float pmin = emin / denom, pmax = emax / denom;
@@ -675,6 +688,9 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         left = __float_as_uint(pmin);
         right = __float_as_uint(pmax) + 1u;
         rounds = 0;
+        // More than top_k elements have e > beta_e: their quotients are >= beta_p, so pivots up to beta_p exceed.  beta_p + 1
+        // need not: many e above beta_e may share the quotient beta_p.  It is evaluated like any other point.
+        const uint32_t sure_to = sure_cnt ? ustar : 0u;
         uint32_t za = max(left, ustar), zb = right;
         uint32_t e0 = 1u, e1 = 0u;                        // none yet
         uint32_t cnt_a = (uint32_t)V, cnt_b = 0u;         // of the sets at za - 1 and zb (estimates until evaluated)
@@ -688,10 +704,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
             const uint32_t pz = (left + right) >> 1, py = (left + pz) >> 1, pw = (pz + right) >> 1;
             // 2 exceeds, 1 neither, 0 passes, -1 unknown
             auto known = [&](uint32_t u) -> int {
-                // More than top_k elements have e > beta_e: their quotients are >= beta_p, so a pivot up to beta_p exceeds.
-                // beta_p + 1 need not: many e above beta_e may share the quotient beta_p.  It is evaluated like any other.
-                if (clamp && sure_cnt && u <= beta_p) return 2;
-                u = max(u, ustar);
+                u = u < sure_to ? 0u : max(u, ustar);
                 return u < za ? 2 : u >= zb ? 0 : (u >= e0 && u <= e1) ? 1 : -1;
             };
             const int c0 = known(py), c1 = known(pz), c2 = known(pw);

@@ -118,3 +118,20 @@ def test_elements_above_the_bound_whose_quotients_tie_with_it(abi, mode, V, low,
         rest[low + near:] = np.float32(x + rng.uniform(0.5, 1.0))
         lg[b] = rng.permutation(rest)
     check_against_oracle(abi, torch.from_numpy(lg), 3, 1.0, k, 1.0, mode, rows=B)
+
+
+@pytest.mark.parametrize("kind,B,V,p,mode", [("head", 32, 1048576, 0.95, 0), ("head", 64, 151936, 0.9, 0), ("head", 64, 151936, 0.95, 0),
+                                             ("head", 128, 50304, 0.95, 0), ("head", 4, 131072, 0.95, 0), ("head", 16, 32000, 0.95, 0),
+                                             ("normal3", 4, 151936, 0.9, 2), ("normal3", 4, 50304, 0.95, 2)])
+def test_lowered_bound_gives_a_list_that_settles_the_row(abi, kind, B, V, p, mode):
+    """Rows whose first list is too thin: a wide head (1 % of the ids raised by 8, nothing else within ten octaves of them)
+    and normal rows.  The list collected again must hold enough and fit, so that no row is searched whole."""
+    if kind == "head":
+        g = torch.Generator(device="cuda").manual_seed(4)
+        lg = torch.randn(B, V, generator=g, device="cuda")
+        ids = torch.stack([torch.randperm(V, generator=g, device="cuda")[:V // 100] for _ in range(B)])
+        lg = lg.scatter_add_(1, ids, torch.full(ids.shape, 8.0, device="cuda")).cpu()
+    else:
+        lg = make_logits(kind, B, V, 41, torch)
+    tr = check_against_oracle(abi, lg, 11, 1.0, -1, p, mode, rows=3)
+    assert [t.path for t in tr] == [0] * B
