@@ -787,9 +787,11 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         return !clamp || left > beta_p;
     };
 
-    // Short rows (V <= 4096, where the bound admits every element to the list) are searched at the reference's own pivots, three a
-    // round: a lane holds an element or two, an evaluation is all exchange, and the placing of the points costs more
-    // than the rounds it saves (B=19, V=1668, top_p 0.3: 18.4 us against 21.2).
+    // Lists of up to 4096 entries (4 per lane) are searched at the reference's own pivots, three a round: a lane holds a few
+    // elements, an evaluation is nearly all exchange, and the placing of the points costs more than the rounds it saves
+    // (this against points of our own: B=19, V=1668, flat: 18.4 and 21.2 us; B=4, V=131072, lists of 1000: 32.5 and 37.0;
+    // B=128, V=50304, lists of 2700: 68.4 and 74.6).  With a line at 16384 instead lists of 8192 (V=8192, flat) gained, 23.7
+    // against 25.5, and N(0, 2^2) rows of V=50304 at top_p 0.9 lost, 93.1 against 89.9.
     //  * frozen: once every element strictly inside (left, right) has one and the same value v, the remaining rounds need
     //    no data: a pivot equal to `left` selects the set of `left`, a pivot in (left, v] the set {p >= v}, a pivot above v
     //    the set of `right`; they are replayed arithmetically.  A closed bracket carries the totals at its upper end.
@@ -1036,7 +1038,7 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
         };
         if (quick != 1) {
             bool ok;
-            if (!whole && V <= 4096) {
+            if (!whole && ncand <= 4096u) {
                 const int m_own = n;
                 auto cand_eval = [&](const float (&f)[4], uint32_t lo, uint32_t hi, uint32_t, float (&m)[4], uint32_t& c01,
                                      uint32_t& c23, uint32_t& mn, uint32_t& mxv) {

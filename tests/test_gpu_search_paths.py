@@ -135,3 +135,12 @@ def test_lowered_bound_gives_a_list_that_settles_the_row(abi, kind, B, V, p, mod
         lg = make_logits(kind, B, V, 41, torch)
     tr = check_against_oracle(abi, lg, 11, 1.0, -1, p, mode, rows=3)
     assert [t.path for t in tr] == [0] * B
+
+
+@pytest.mark.parametrize("mode", [0, 2, 6])           # the planner's choice, streaming, exact search only
+@pytest.mark.parametrize("kind,V,p", [("uniform", 4096, 0.5), ("uniform", 4100, 0.5), ("coarse", 4096, 0.6), ("coarse", 4100, 0.6),
+                                      ("normal3", 20480, 0.9), ("normal3", 32000, 0.9), ("normal3", 50304, 0.9)])
+def test_list_lengths_around_the_line_between_the_two_searches(abi, mode, kind, V, p):
+    """Lists of 513 to about 7000 entries, on both sides of the 4096 up to which the reference's own pivots are evaluated."""
+    tr = check_against_oracle(abi, make_logits(kind, 12, V, 51, torch), 13, 1.0, -1, p, mode, rows=12)
+    assert any(t.path == 0 and t.ncand > 512 for t in tr)
