@@ -27,6 +27,8 @@ struct Params {
     int cand_slots;          // float4 slots per lane of the candidate buffer (shared-memory variant)
     float scale, top_p, presence, repetition, decay;
     const struct RowArgs* rows;   // per-row parameters (ROWP kernels only), else null
+    const int* route;        // per-row parameters: word the rows' settings decide (1: some row searches widely), or null
+    int route_is;            // the kernel runs only if the word holds this
     float* out_prob;         // optional B: probability of the sampled id (ROWP kernels only)
     float* out_kept;         // optional B: kept probability mass the id was drawn from (ROWP kernels only)
     int quick;               // 1: try the search on integer masses first; 0 (test instrumentation): exact search only

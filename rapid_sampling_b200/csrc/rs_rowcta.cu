@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
     int a_kind = p.kind, a_top_k = p.top_k, a_sel_rank = p.sel_rank;
     float a_scale = p.scale, a_top_p = p.top_p;
     if (p.rows) {   // this row's own normalised parameters
+        if (p.route && *p.route != p.route_is) return;      // the other kernel serves this call
         const RowArgs ra = p.rows[b];
         a_kind = ra.kind; a_top_k = ra.top_k; a_sel_rank = ra.sel_rank; a_scale = ra.scale; a_top_p = ra.top_p;
     }

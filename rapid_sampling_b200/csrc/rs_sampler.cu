@@ -60,6 +60,12 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     // have been set up while its predecessor ran -- nothing in global memory is touched before the predecessor is
     // complete and visible.
     grid_dependents_may_launch();
+    if (ROWP && p.route && __ldcg(p.route) != p.route_is) {
+        // The other sampler kernel, this one's predecessor, serves the call.  The word was written by the predecessor of that
+        // one, which has completed.  One CTA stays until the predecessor is done: this grid must not end before it.
+        if (blockIdx.x == 0) grid_dependency_wait();
+        return;
+    }
     grid_dependency_wait();
     // per-call parameters, or (ROWP) this row's own
     int a_kind = p.kind, a_top_k = p.top_k, a_sel_rank = p.sel_rank;
@@ -1273,11 +1279,10 @@ __global__ void selftest_wait_kernel(int* status, int* status_mirror, uint32_t p
 
 // Per-row parameters: the host functions' checks and remaps (sampling.cu:458-486, :982-1011) applied to every row
 // on the device.  A temperature outside [0.001, 1000] cannot raise here; the row is sampled at temperature 1 and
-// the status word reports RS_ERR_TEMPERATURE.
-__global__ void row_args_kernel(int B, int V, const float* temperature, const int* top_k, const float* top_p, int rep,
-                                int allow_candidates, RowArgs* out, int* status, int* status_mirror) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
+// the status word reports RS_ERR_TEMPERATURE.  Returns whether the row searches widely: it has a top_p but no top_k, or a
+// top_k too large for the candidate bound.
+__device__ __forceinline__ bool row_args_one(int b, int V, const float* temperature, const int* top_k, const float* top_p, int rep,
+                                             int allow_candidates, RowArgs* out, int* status, int* status_mirror) {
     float tmp = temperature ? temperature[b] : 1.0f;
     long long k = top_k ? top_k[b] : -1;
     float pp = top_p ? top_p[b] : 1.0f;
@@ -1303,6 +1308,18 @@ __global__ void row_args_kernel(int B, int V, const float* temperature, const in
     r.sel_rank = sel;
     r.pad0 = 0; r.pad1 = r.pad2 = 0.f;
     out[b] = r;
+    return !(k >= V && pp >= 1.0f) && (sel == 0 || k >= V);
+}
+// route (calls of one block only): whether any row does
+__global__ void row_args_kernel(int B, int V, const float* temperature, const int* top_k, const float* top_p, int rep,
+                                int allow_candidates, RowArgs* out, int* status, int* status_mirror, int* route) {
+    int wide = 0;
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x)
+        wide |= row_args_one(b, V, temperature, top_k, top_p, rep, allow_candidates, out, status, status_mirror) ? 1 : 0;
+    if (route) {
+        wide = __syncthreads_or(wide);
+        if (threadIdx.x == 0) *route = wide ? 1 : 0;
+    }
 }
 
 // ------------------------------------------------------------------ host side -------------
@@ -1367,7 +1384,8 @@ static int launch_typed(const Params& p, int smem, cudaStream_t stream, DeviceIn
     // Early scheduling pays for small grids (measured: B=1 24.7 -> 23.1 us, B=4 53.2 -> 51.3 us per back-to-back call).  A
     // grid that fills most of the GPU is better placed on an empty one: its CTAs would take whatever slots the
     // predecessor left free and end up unevenly spread (B=64, 512 CTAs: 36.6 -> 39.9 us).
-    if (g_dependent_launch.load() && (long long)p.B * C * 2 <= di.sms) {   // the kernel waits for its predecessor itself
+    // (p.route: the predecessor is the other sampler kernel of the same call; one of the two returns at once.)
+    if (g_dependent_launch.load() && ((long long)p.B * C * 2 <= di.sms || p.route)) {   // the kernel waits for its predecessor itself
         at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[na].val.programmaticStreamSerializationAllowed = 1;
         na++;
@@ -1534,6 +1552,8 @@ static int sample_impl(const void* logits, int dtype, int64_t B, int64_t T, int6
     p.dbg_probs = dbg_probs;
     p.dbg_trace = dbg_trace;
     p.rows = nullptr;
+    p.route = nullptr;
+    p.route_is = 0;
     p.out_prob = nullptr;
     p.out_kept = nullptr;
     p.quick = (g_path_override.load() < 5) ? 1 : 0;
@@ -1598,26 +1618,38 @@ static int sample_rows_impl(const void* logits, int dtype, int64_t B, int64_t T,
     // rows differ in top_k: the candidate buffer takes the widest size
     const bool allow_cand = g_path_override.load() != 1;
     Plan pl = make_plan(*di, B, (int)V, allow_cand ? 8 : 0, allow_cand ? 4 : 0, workspace_bytes - rab);
-    {   // large batches: one CTA per row, as for per-call parameters
+    // Large batches: one CTA per row, as for per-call parameters.  For long rows that hangs on their settings: a row without a
+    // top_k, or with a large one, searches much of itself, and the call lasts as long as its slowest row.  The settings are
+    // on the device, so the kernel that normalises them decides, both sampler kernels are launched, and one of them returns
+    // at once.  One CTA per row / streaming / this choice, us a call (K: every row has a top_k; M: one in five has none):
+    //   f32 B=160 V=16384    K 26.5  38.4  28.1   M  88.5  49.3  48.1        bf16 B=512 V=32768   K 54.1  88.3  55.2   M 165.4 108.5 109.6
+    //   f32 B=256 V=65536    K 46.1  56.4  47.8   M 223.2  90.1  94.3        f32  B=256 V=151936  K 75.0  87.1  76.6   M 437.8 169.0 174.5
+    //   f32 B=112 V=65536    K 29.6  33.8  31.0   M 136.4  62.6  65.6        pen. B=256 V=16384   K 38.4  54.7  40.2   M 109.3  68.1  66.8
+    //   pen. B=256 V=65536   K 78.1  81.4  82.4   M 269.9 117.7 129.0        pen. B=512 V=32768   K 92.0 108.7 103.9   M 203.0 128.8 134.3
+    // The choice is left out, and such calls stream, where it gains no more than the second launch costs: beyond 16384 columns
+    // with penalties, or with no more rows than SMs.  Up to 8192 columns a whole-row search is cheap, and the rows always have a
+    // CTA each: bf16 B=256 V=8192 K 28.5  48.5, M 47.5  48.4; B=512 K 43.5  82.6, M 68.7  85.5.  (A small top_p without a top_k
+    // counts as wide, though its list may be short: bf16, top_p 0.3 or 0.5, B=256 V=65536 N(0, 2.5^2) 203.0  97.4, 1 % of the ids
+    // raised by 8 121.4  74.2, B=512 V=32768 147.2  128.0 and 55.7  88.8.)
+    bool either = false;
+    {
         const int mode = g_path_override.load();
         const bool eligible = workspace_bytes - rab >= ws_bytes(B, V);
-        // ... if the rows are short: among rows that bring their own settings some have no top_k and search much of their row,
-        // and the call lasts as long as they do (a mix of settings, one CTA per row against streaming: B=133 V=106860 bf16
-        // 200.7 / 90.2 us, B=256 V=65536 with penalties 279.0 / 123.7, B=300 V=16384 bf16 95.7 / 64.9)
-        const bool wanted = (mode == 4 || mode == 5) ||
-                            ((mode == 0 || mode == 6) && g_cluster_override.load() == 0 && !pl.smem && B >= kRowCtaMinBatch && V <= 8192);
-        if (eligible && wanted) {
+        const bool large = (mode == 0 || mode == 6) && g_cluster_override.load() == 0 && !pl.smem && B >= kRowCtaMinBatch;
+        if (eligible && (mode == 4 || mode == 5 || (large && V <= 8192))) {
             pl.rowcta = true;
             pl.ws = ws_bytes(B, V);
         }
+        either = eligible && large && V > 8192 && (V <= 16384 || (!penalties && B > di->sms));
     }
     if (workspace_bytes < pl.ws + rab) return RS_ERR_WORKSPACE;
     if (pl.smem && pl.C != 8 && pl.C != 16) return RS_ERR_LIMIT;   // forced widths exist for the per-call entry only
 
     cudaStream_t st = (cudaStream_t)stream;
     RowArgs* rows = (RowArgs*)((char*)workspace + 256);
-    row_args_kernel<<<(unsigned)((B + 127) / 128), 128, 0, st>>>((int)B, (int)V, temperature, top_k, top_p, penalties ? 1 : 0,
-                                                               allow_cand ? 1 : 0, rows, (int*)workspace, di->mirror);
+    int* route = either ? (int*)workspace + 16 : nullptr;      // (in the 256 bytes of the status word)
+    row_args_kernel<<<either ? 1u : (unsigned)((B + 127) / 128), either ? 1024 : 128, 0, st>>>(
+        (int)B, (int)V, temperature, top_k, top_p, penalties ? 1 : 0, allow_cand ? 1 : 0, rows, (int*)workspace, di->mirror, route);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "launch(row_args)");
     g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -1636,6 +1668,8 @@ static int sample_rows_impl(const void* logits, int dtype, int64_t B, int64_t T,
     p.dbg_probs = nullptr;
     p.dbg_trace = nullptr;
     p.rows = rows;
+    p.route = route;
+    p.route_is = 0;
     p.out_prob = out_prob;
     p.out_kept = out_kept;
     p.quick = (g_path_override.load() < 5) ? 1 : 0;
@@ -1650,14 +1684,15 @@ static int sample_rows_impl(const void* logits, int dtype, int64_t B, int64_t T,
     p.decay = (float)decay;
     p.sel_rank = 0;
     p.cand_slots = pl.cand_slots;
-    if (pl.rowcta) {
+    if (pl.rowcta || either) {
         const int budget = (B <= di->sms) ? di->smem_optin : (di->smem_sm / 2 - 1024);
         const int lpt = (B <= di->sms) ? 2 : 4;
         const RowCtaPlan rp = rowcta_plan((int)V, penalties != nullptr, allow_cand ? 8 : 0, lpt, budget);
-        rc = rowcta_launch(p, rp, lpt, st, di->smem_optin, g_dependent_launch.load() != 0 && B * 2 <= di->sms);
+        rc = rowcta_launch(p, rp, lpt, st, di->smem_optin, !either && g_dependent_launch.load() != 0 && B * 2 <= di->sms);
         if (rc == RS_OK) g_launches.fetch_add(1, std::memory_order_relaxed);
         else if (rc == RS_ERR_CUDA) return cuda_fail(cudaGetLastError(), "launch(rowcta, per-row)");
-        return rc;
+        if (rc != RS_OK || !either) return rc;
+        p.route_is = 1;
     }
     if (!pl.smem) return launch_rows<8, false>(p, kSlabOff + pl.cand_slots * (kLanes / 8) * 16, st, *di);
     const int smem = smem_need((int)V, pl.C, pl.cand_slots);
@@ -1731,6 +1766,8 @@ static int sample_static_impl(const float* logits, int64_t B, int64_t T, int64_t
     p.dbg_probs = nullptr;
     p.dbg_trace = nullptr;
     p.rows = nullptr;
+    p.route = nullptr;
+    p.route_is = 0;
     p.out_prob = nullptr;
     p.out_kept = nullptr;
     p.quick = (g_path_override.load() < 5) ? 1 : 0;

@@ -48,7 +48,7 @@ def test_rows_equal_one_row_reference_calls(ref, B, V, kind, rep):
             assert torch.equal(pen_o, pen_r)
 
 
-@pytest.mark.parametrize("B", [12, 160])     # the larger batch runs one CTA per row
+@pytest.mark.parametrize("B", [12, 160])     # the larger batch has rows without a top_k: streaming clusters
 def test_rows_bf16_logits_and_neutral_defaults(ref, B):
     import rapid_sampling_b200 as rs
     V = 65536
@@ -67,7 +67,7 @@ def test_rows_bf16_logits_and_neutral_defaults(ref, B):
     assert torch.equal(a, b_) and torch.equal(st_a, st_b)
 
 
-@pytest.mark.parametrize("B", [9, 153])      # the larger batch runs one CTA per row
+@pytest.mark.parametrize("B", [9, 153])      # the larger batch has rows without a top_k: streaming clusters
 def test_rows_probability_and_kept_mass(B):
     import rapid_sampling_b200 as rs
     from oracle import cpu_ref
@@ -111,7 +111,7 @@ def test_rows_bad_temperature_sets_status_and_spares_other_rows(abi):
                             None, None, ws.data_ptr(), 256, abi.stream()) == abi.abi.RS_ERR_WORKSPACE
 
 
-@pytest.mark.parametrize("B", [12, 300])     # the larger batch runs one CTA per row
+@pytest.mark.parametrize("B", [12, 300])     # the larger batch has rows without a top_k: streaming clusters
 def test_rows_probability_is_taken_before_the_penalty_update(B):
     """With penalties, the reported probability of the sampled id must come from the penalties as they were BEFORE
     the call (the same values the softmax ran on), on every call of a chain."""
@@ -131,3 +131,60 @@ def test_rows_probability_is_taken_before_the_penalty_update(B):
             d = cpu_ref.distribution(lg[b:b + 1], float(t[b]), int(k[b]), float(p[b]), penalties=before[b:b + 1])
             want = float(d["probs"][0, ids[b]])
             assert abs(float(prob[b]) - want) <= 1e-5 * want + 1e-12, (call, b, float(prob[b]), want)
+
+
+# every row has a top_k that the candidate bound takes, or no cutoff at all; and the same with one wide row
+NARROW = [(1.0, 50, 0.9), (0.8, 20, 1.0), (1.3, 1, 1.0), (0.7, 254, 0.95), (1.0, 10, 0.0), (2.0, 0, 1.0), (0.6, 100, 0.8)]
+
+
+@pytest.mark.parametrize("wide", [None, (1.0, -1, 0.9), (0.9, 255, 1.0)])
+@pytest.mark.parametrize("B,V,kind,dtype,rep", [(112, 8192, "normal3", "f32", False), (130, 8188, "peaked", "bf16", True),
+                                                (112, 8196, "normal3", "bf16", False), (160, 16384, "peaked", "f32", True),
+                                                (1030, 8452, "normal3", "f16", False), (149, 16388, "peaked", "bf16", False)])
+def test_large_batches_equal_one_row_calls_on_either_kernel(abi, B, V, kind, dtype, rep, wide):
+    """Ids, states, penalties, and which kernel the settings chose: one CTA per row if none of the rows is wide (and always
+    up to 8192 columns), streaming clusters otherwise.  The last row's setting changes between calls recorded in one graph,
+    so the choice is made anew on each replay."""
+    lg = make_logits(kind, B, V, 61, torch).cuda().to({"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dtype])
+    settings = [NARROW[b % len(NARROW)] for b in range(B)]
+    t, k, p = (torch.tensor([s[i] for s in settings], dtype=d, device="cuda") for i, d in enumerate((torch.float32, torch.int32, torch.float32)))
+    L, A = abi.L, abi.abi
+    code = {"f32": A.RS_DTYPE_F32, "bf16": A.RS_DTYPE_BF16, "f16": A.RS_DTYPE_F16}[dtype]
+    ws = torch.zeros(L.rs_rows_workspace_bytes(B, V), dtype=torch.uint8, device="cuda")
+    out = torch.empty(B, dtype=torch.int32, device="cuda")
+    st, st_one = abi.setup_rand(14, B), abi.setup_rand(14, B)
+    gen = torch.Generator().manual_seed(2)
+    pen = (torch.rand(B, V, generator=gen) * (torch.rand(B, V, generator=gen) < 0.01)).cuda() if rep else None
+    pen_one = pen.clone() if rep else None
+
+    def call():
+        rc = L.rs_sample_rows(lg.data_ptr(), code, B, 1, V, pen.data_ptr() if rep else None, st.data_ptr(), out.data_ptr(), t.data_ptr(),
+                              k.data_ptr(), p.data_ptr(), 0.1, 0.2, 0.9, None, None, ws.data_ptr(), ws.numel(), abi.stream())
+        assert rc == 0, A.status_string(rc)
+
+    def check(last):
+        rows = sorted({0, 1, 2, 3, 4, 5, 6, B // 2, B - 2, B - 1})
+        for b in rows:
+            s = last if b == B - 1 and last else settings[b]
+            one = abi.sample(lg[b:b + 1], st_one[64 * b:64 * b + 64], float(np.float32(s[0])), s[1], float(np.float32(s[2])),
+                             penalties=pen_one[b:b + 1] if rep else None, presence=0.1, repetition=0.2, decay=0.9)
+            assert int(one[0]) == int(out[b]), (b, s)
+            assert torch.equal(st_one[64 * b:64 * b + 64], st[64 * b:64 * b + 64])
+            if rep:
+                assert torch.equal(pen_one[b], pen[b])
+        if V > 8192:
+            assert int(ws.view(torch.int32)[16]) == (1 if last else 0)
+
+    call()
+    torch.cuda.synchronize()
+    check(None)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call()
+    for last in (wide, None, wide):
+        s = last or settings[B - 1]
+        t[B - 1], k[B - 1], p[B - 1] = s
+        g.replay()
+        torch.cuda.synchronize()
+        check(last)
+    assert L.rs_device_status(ws.data_ptr(), abi.stream()) == 0
