@@ -111,33 +111,39 @@ __device__ __forceinline__ void f_block_sums30(float (&v)[30], float* sh /* [32]
 }
 
 // The staged passes are bound by the latency of their loads (a row stays with one CTA, because its sums are fixed chains
-// per thread) and, for elements that matter, by the exponential and the division.  vp_for_each fetches U elements of a
-// thread's chain ahead and calls body(i, x) for i = t, t + 1024, ... in that order.
+// per thread) and, for elements that matter, by the exponential and the division.  vp_fetch loads U elements of a thread's
+// chain i = t, t + 1024, ... ahead (those beyond the row hold anything); vp_for_each calls body(i, x) for all of them in
+// that order.
+template <int U>
+__device__ __forceinline__ void vp_fetch(const VpRow& r, int i0, float scale, float (&x)[U]) {
+    float q[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int i = i0 + u * kVpThreads;
+        x[u] = (i < r.n) ? r.logits[i] : 0.f;
+    }
+    if (r.penalties) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = i0 + u * kVpThreads;
+            q[u] = (i < r.n) ? r.penalties[i] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) x[u] = sanitize((sanitize(x[u]) - q[u]) * scale);
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; u++) x[u] = sanitize(x[u] * scale);
+    }
+}
 template <int U, class F>
 __device__ __forceinline__ void vp_for_each(const VpRow& r, float scale, F&& body) {
     for (int i0 = (int)threadIdx.x; i0 < r.n; i0 += U * kVpThreads) {
-        float l[U], q[U];
+        float x[U];
+        vp_fetch(r, i0, scale, x);
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int i = i0 + u * kVpThreads;
-            l[u] = (i < r.n) ? r.logits[i] : 0.f;
-        }
-        if (r.penalties) {
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int i = i0 + u * kVpThreads;
-                q[u] = (i < r.n) ? r.penalties[i] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) l[u] = sanitize((sanitize(l[u]) - q[u]) * scale);
-        } else {
-#pragma unroll
-            for (int u = 0; u < U; u++) l[u] = sanitize(l[u] * scale);
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int i = i0 + u * kVpThreads;
-            if (i < r.n) body(i, l[u]);
+            if (i < r.n) body(i, x[u]);
         }
     }
 }
@@ -147,29 +153,35 @@ __device__ __forceinline__ float vp_cut(uint32_t p_bits, float denom) {
     return p_bits < 0x01000000u ? -INFINITY : log2f(__uint_as_float(p_bits) * denom) - 0.05f;
 }
 
-// Calls body(x - max) for the elements at or above the cut, in chain order.  They are few: noted first, so that the loads run
-// ahead of a loop that holds neither the exponential nor the division (a thread that notes more than kVpNoted sends the
-// whole block through the row once more).
-constexpr int kVpNoted = 8;      // 32 KiB of shared memory
+// Calls body(x - max) for the elements at or above the cut, in chain order.  Mostly they are few: they are noted first, so
+// that the loads run ahead of a loop that holds neither the exponential and the division nor the body's sums.  A warp of
+// which some thread has noted more than kVpNoted weighs what it has and goes on in turns of loads, notes and weighing: it
+// weighs as often as its fullest thread has noted, not once for nearly every element.  (B=32, 131072 columns N(0, 3^2), top_p
+// 0.95, where most threads note 8 to 20: starting the row over without notes when a thread was full took 1279 us a call.)
+constexpr int kVpAhead = 16, kVpNoted = 8;
+constexpr size_t kVpNoteBytes = (size_t)(kVpNoted + kVpAhead) * kVpThreads * sizeof(float);      // 96 KiB; one CTA per SM anyway
 template <class F>
 __device__ __forceinline__ void vp_select(const VpRow& r, float scale, float mx, float cut, float* s_list, F&& body) {
-    bool noted = cut > -INFINITY;
-    if (noted) {
-        int m = 0;
-        vp_for_each<16>(r, scale, [&](int, float x) {
-            if (x - mx >= cut) {
-                if (m < kVpNoted) s_list[m * kVpThreads + (int)threadIdx.x] = x - mx;
-                m++;
-            }
-        });
-        noted = __syncthreads_or(m > kVpNoted ? 1 : 0) == 0;
-        if (noted)
-            for (int i = 0; i < m; i++) body(s_list[i * kVpThreads + (int)threadIdx.x]);
+    float* mine = s_list + threadIdx.x;
+    int m = 0, base = 0;
+    auto note = [&]() {
+        float x[kVpAhead];
+        vp_fetch(r, base + (int)threadIdx.x, scale, x);
+#pragma unroll
+        for (int u = 0; u < kVpAhead; u++)
+            if (x[u] - mx >= cut && base + (int)threadIdx.x + u * kVpThreads < r.n) mine[m++ * kVpThreads] = x[u] - mx;
+        base += kVpAhead * kVpThreads;
+    };
+    while (base < r.n && !__any_sync(0xffffffffu, m > kVpNoted)) note();
+    for (int i = 0; i < m; i++) body(mine[i * kVpThreads]);
+    m = 0;
+    while (base < r.n) {
+        note();
+        if (base >= r.n || __any_sync(0xffffffffu, m > kVpNoted)) {
+            for (int i = 0; i < m; i++) body(mine[i * kVpThreads]);
+            m = 0;
+        }
     }
-    if (!noted)
-        vp_for_each<8>(r, scale, [&](int, float x) {
-            if (x - mx >= cut) body(x - mx);
-        });
 }
 
 __global__ void __launch_bounds__(kVpThreads) vp_max_kernel(const float* logits, long long row_stride, float* penalties,
@@ -240,7 +252,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_round_kernel(const float* logit
                                                               int n, float scale, const float* gmax, const float* gsum,
                                                               const float* tallies, int B, int round, float top_k,
                                                               float top_p, float* out /* [B][15][2] */) {
-    __shared__ float s_list[kVpNoted * kVpThreads];
+    extern __shared__ float s_list[];      // kVpNoteBytes
     __shared__ float sh[32 * 32 + 32];
     const int b = blockIdx.x, t = threadIdx.x;
     const VpRow r = vp_row(logits, row_stride, penalties, n, b);
@@ -297,7 +309,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_tally_kernel(const float* logit
                                                               int n, float scale, const float* gmax, const float* gsum,
                                                               const float* tallies, int B, int rounds, float top_k,
                                                               float top_p, float* out /* [B][4] */) {
-    __shared__ float s_list[kVpNoted * kVpThreads];
+    extern __shared__ float s_list[];      // kVpNoteBytes
     __shared__ float sh[32 * 3 + 3];
     const int b = blockIdx.x;
     const VpRow r = vp_row(logits, row_stride, penalties, n, b);
@@ -337,7 +349,7 @@ __global__ void __launch_bounds__(kVpThreads) vp_weight_kernel(const float* logi
                                                                const float* tallies, int B, int rounds, float top_k,
                                                                float top_p, int use_p, const float* gtally, int rank,
                                                                int world, float* out /* [B][world] */) {
-    __shared__ float s_list[kVpNoted * kVpThreads];
+    extern __shared__ float s_list[];      // kVpNoteBytes
     __shared__ float sh[32];
     const int b = blockIdx.x;
     const VpRow r = vp_row(logits, row_stride, penalties, n, b);
@@ -1126,6 +1138,16 @@ int rs_vp_stage(const rs_vp_call* c, int32_t stage, int32_t round) {
     const long long stride = (long long)T * n;
     cudaStream_t st = (cudaStream_t)c->stream;
     const unsigned grid = (unsigned)B;
+    if (stage == RS_VP_ROUND || stage == RS_VP_TALLY || stage == RS_VP_WEIGHT) {
+        static bool attr_done_s[64] = {};     // per device
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return RS_ERR_CUDA;
+        if (!attr_done_s[dev]) {
+            for (const void* k : {(const void*)vp_round_kernel, (const void*)vp_tally_kernel, (const void*)vp_weight_kernel})
+                if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVpNoteBytes) != cudaSuccess) return RS_ERR_CUDA;
+            attr_done_s[dev] = true;
+        }
+    }
     switch (stage) {
         case RS_VP_MAX:
             vp_max_kernel<<<grid, kVpThreads, 0, st>>>(lg, stride, c->penalties, (int)n, scale, ws + l.gmax);
@@ -1135,17 +1157,17 @@ int rs_vp_stage(const rs_vp_call* c, int32_t stage, int32_t round) {
             break;
         case RS_VP_ROUND:
             if (round < 0 || round >= RS_VP_ROUNDS) return RS_ERR_LIMIT;
-            vp_round_kernel<<<grid, kVpThreads, 0, st>>>(lg, stride, c->penalties, (int)n, scale, ws + l.gmax, ws + l.gsum,
+            vp_round_kernel<<<grid, kVpThreads, kVpNoteBytes, st>>>(lg, stride, c->penalties, (int)n, scale, ws + l.gmax, ws + l.gsum,
                                                          ws + l.tallies, (int)B, round, fk, fp,
                                                          ws + l.tallies + (size_t)round * B * kVpPivots * 2);
             break;
         case RS_VP_TALLY:
-            vp_tally_kernel<<<grid, kVpThreads, 0, st>>>(lg, stride, c->penalties, (int)n, scale, ws + l.gmax, ws + l.gsum,
+            vp_tally_kernel<<<grid, kVpThreads, kVpNoteBytes, st>>>(lg, stride, c->penalties, (int)n, scale, ws + l.gmax, ws + l.gsum,
                                                          ws + l.tallies, (int)B, RS_VP_ROUNDS, fk, fp, ws + l.gtally);
             break;
         case RS_VP_WEIGHT:
             if (cudaMemsetAsync(ws + l.weights, 0, (size_t)B * c->world * sizeof(float), st) != cudaSuccess) return RS_ERR_CUDA;
-            vp_weight_kernel<<<grid, kVpThreads, 0, st>>>(lg, stride, c->penalties, (int)n, scale, ws + l.gmax, ws + l.gsum,
+            vp_weight_kernel<<<grid, kVpThreads, kVpNoteBytes, st>>>(lg, stride, c->penalties, (int)n, scale, ws + l.gmax, ws + l.gsum,
                                                           ws + l.tallies, (int)B, RS_VP_ROUNDS, fk, fp, use_p, ws + l.gtally,
                                                           c->rank, c->world, ws + l.weights);
             break;

@@ -335,3 +335,44 @@ def test_lm_head_tile_hook_through_the_driver(abi):
         got = h.sample(shard, st_h, 0.8, 50, 0.9, max_from_tiles=True).clone()
         assert h.last_protocol == "fast"
         assert torch.equal(got, want) and torch.equal(st_a, st_h)
+
+
+@pytest.mark.parametrize("kind,V,N,p,penalised", [("normal3", 135172, 1, 0.95, False), ("normal3", 135172, 1, 0.95, True),
+                                                  ("uniform", 8196, 1, 0.9, True), ("normal3", 60008, 2, 0.95, False),
+                                                  ("uniform", 1028, 1, 0.5, False), ("peaked", 40012, 1, 0.99, True),
+                                                  ("coarse", 20488, 2, 0.7, False)])
+def test_staged_protocol_walks_the_kept_columns_in_order(abi, kind, V, N, p, penalised):
+    """The staged protocol names the first kept column whose running weight reaches u times the total, u being the row's draw:
+    against a float64 walk in column order.  Threads that note more elements than fit and weigh them early (flat rows and
+    normal ones), shards that are no multiple of 1024 columns, and of more than the 131072 whose totals the pick holds at
+    once, with a third of the weight behind them.  Slack: fp32 sums of up to 135172 terms, and one boundary element."""
+    from rapid_sampling_b200.vocab_parallel import VocabParallelSampler
+    from oracle import c_oracle as co
+    B = 8
+    full = make_logits(kind, B, V, 15, torch)
+    if V > 131072:
+        full[:, 131072:] += 3.0
+    samplers = [VocabParallelSampler(B, V, r, N) for r in range(N)]
+    shards = [full[:, s.col0:s.col0 + s.V_local].contiguous().cuda() for s in samplers]
+    states = [abi.setup_rand(19, B) for _ in range(N)]
+    gen = torch.Generator().manual_seed(5)
+    pen = torch.rand(B, V, generator=gen) * (torch.rand(B, V, generator=gen) < 0.3) if penalised else None
+    pens = [pen[:, s.col0:s.col0 + s.V_local].contiguous().cuda() for s in samplers] if penalised else None
+    behind = 0
+    for call in range(6):
+        st = states[0].cpu().numpy().copy()
+        ids = emulated_sample(samplers, shards, states, 0.9, -1, p, pens, fast=False)
+        torch.cuda.synchronize()
+        got = ids[0].cpu().numpy()
+        d = cpu_ref.distribution(full, 0.9, -1, p, penalties=pen)
+        for b in range(B):
+            cum = np.cumsum(d["weights"][b].numpy())
+            target = co.uniform(co.draw4(st, b)[0]) * cum[-1]
+            slack = 2e-5 * cum[-1] + 2 * float(d["v"][b])
+            lo = cum[got[b] - 1] if got[b] > 0 else 0.0
+            assert lo - slack <= target <= cum[got[b]] + slack, (call, b, got[b], lo, target, cum[got[b]])
+            assert float(d["weights"][b][got[b]]) > 0 or abs(float(d["probs"][b][got[b]]) - float(d["v"][b])) <= 1e-5 * float(d["v"][b])
+            behind += int(got[b] >= 131072)
+        if penalised:
+            pen = torch.cat([x.cpu() for x in pens], dim=1)
+    assert V <= 131072 or behind >= 5
