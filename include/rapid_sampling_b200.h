@@ -191,7 +191,8 @@ enum { RS_VP_MAX = 0, RS_VP_SUM = 1, RS_VP_ROUND = 2, RS_VP_TALLY = 3, RS_VP_WEI
         * elements), VPF_EXTRACT (bound chosen from the reduced histogram), VPF_COMPACT, all-gather, VPF_FINISH.
         * Regions from rs_vp_fast_layout (floats): [0] stat1 B*S (all-reduce MAX),
         * [1] stat2 B*S*[10] (all-reduce SUM), [2] send list B*Lmax*2 + [3] send counts B (all-gather into [4] and [5]),
-        * [6] ids + 1 (int32 B), [7] valid flags (int32 B; a 0 means: repeat the call with the staged protocol),
+        * [6] ids + 1 (int32 B), [7] valid flags (int32 B, one per row, and behind them one for the call, 0 if any row's is;
+        * a 0 means: repeat the call with the staged protocol -- ids of rows flagged 1 stand, but no state was advanced),
         * [8] = S, [9] = Lmax.  RS_VP_PENALTY with round = 1 applies the fast protocol's ids. */
        RS_VPF_MAX = 10, RS_VPF_SUM = 11, RS_VPF_COMPACT = 12, RS_VPF_FINISH = 13, RS_VPF_ADVANCE = 14, RS_VPF_EXTRACT = 15 };
 typedef struct rs_vp_call {

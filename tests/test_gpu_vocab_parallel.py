@@ -376,3 +376,32 @@ def test_staged_protocol_walks_the_kept_columns_in_order(abi, kind, V, N, p, pen
         if penalised:
             pen = torch.cat([x.cpu() for x in pens], dim=1)
     assert V <= 131072 or behind >= 5
+
+
+@pytest.mark.parametrize("N", [1, 2])
+def test_only_rows_that_could_not_be_listed_are_flagged(abi, N):
+    """A flat row overflows its lists and voids the call (nothing is advanced), but the per-row flags name that row alone, and
+    the ids of the other rows are those of a call without it."""
+    from rapid_sampling_b200.vocab_parallel import VocabParallelSampler
+    V, flat = 65536, [1, 4]
+    B = 6
+    full = make_logits("peaked", B, V, 23, torch)
+    full[flat] = torch.rand(len(flat), V, generator=torch.Generator().manual_seed(1))
+    good = [b for b in range(B) if b not in flat]
+
+    def fast_ids(rows):
+        samplers = [VocabParallelSampler(len(rows), V, r, N) for r in range(N)]
+        shards = [full[rows][:, s.col0:s.col0 + s.V_local].contiguous().cuda() for s in samplers]
+        whole = abi.setup_rand(31, B)
+        states = [torch.cat([whole[64 * b:64 * b + 64] for b in rows]) for _ in range(N)]
+        emulated_sample(samplers, shards, states, 1.0, -1, 0.5)
+        torch.cuda.synchronize()
+        return emulated_sample.last, [(s.f_ids.clone() - 1, s.f_valid.clone()) for s in samplers]
+
+    last, got = fast_ids(list(range(B)))
+    assert last == "staged"
+    last, want = fast_ids(good)
+    assert last == "fast"
+    for (ids, valid), (ids_good, _) in zip(got, want):
+        assert valid.tolist() == [0 if b in flat else 1 for b in range(B)]
+        assert ids[good].tolist() == ids_good.tolist()
