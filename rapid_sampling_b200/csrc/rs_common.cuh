@@ -298,10 +298,10 @@ __device__ __forceinline__ float4 scaled4_rep(float4 l, float4 q, float scale) {
 // Correctly rounded quotients by one denominator (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. Res. Dev. 34(1), 1990): y is the correctly rounded 1/b; the first correction makes q a
 // neighbour of a/b (what it rounds is within 1.5 ulp * 2^-24 of a/b), and for such a q with an exact remainder the second
-// one yields the rounded quotient.  Remainders are exact and nothing underflows for a >= kDivMin (a multiple of a's last
-// place times 2^-24 stays normal); a = 0 gives 0.  Five fused operations instead of a call of the general division
+// one yields the rounded quotient.  Remainders are exact and nothing underflows for a >= kDivMin = 2^-78 (they are multiples
+// of a's last place times 2^-24, that is of 2^-125 or more); a = 0 gives 0.  Five fused operations instead of a call of the general division
 // with its reciprocal and its range test per element; the same bits (tests/test_division.py repeats the steps exactly).
-constexpr float kDivMin = 1.0e-24f;
+constexpr float kDivMin = 3.30872245e-24f;
 __device__ __forceinline__ float div_by(float a, float b, float y) {
     float q = a * y;
     q = fmaf(fmaf(-q, b, a), y, q);

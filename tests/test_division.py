@@ -26,8 +26,11 @@ def fma(a, b, c):
 
 def div_by(a, b, y):
     q = rn(Fraction(float(a)) * Fraction(float(y)))
-    q = fma(fma(-q, b, a), y, q)
-    return fma(fma(-q, b, a), y, q)
+    for _ in range(2):
+        r = fma(-q, b, a)
+        assert r == 0 or abs(r) >= np.float32(2.0 ** -126), (a, b)      # no remainder is subnormal
+        q = fma(r, y, q)
+    return q
 
 
 def test_two_corrections_give_the_rounded_quotient():
@@ -41,6 +44,6 @@ def test_two_corrections_give_the_rounded_quotient():
             m = Fraction(float(np.float32(np.exp2(g.uniform(-60, -20))))) * (1 + Fraction(1, 2 ** 24))
             a = rn(m * Fraction(float(b)))
         else:
-            a = np.float32(np.exp2(g.uniform(-79, 0)))
-        assert a >= np.float32(1e-24)
+            a = np.float32(2.0 ** -78) if i % 50 == 0 else np.float32(np.exp2(g.uniform(-78, 0)))      # down to kDivMin
+        assert a >= np.float32(2.0 ** -78)
         assert div_by(a, b, y) == rn(Fraction(float(a)) / Fraction(float(b))), (a, b)
