@@ -47,8 +47,9 @@ typedef struct rs_trace {
     uint32_t ncand;  /* elements on the candidate list */
     uint32_t t_ns[10]; /* ns since kernel entry of the owner CTA's thread 0 at: 1 row resident, 2 pass 1, 3 exchange,
                           4 pass 2, 5 exchange, 6 search+recount, 7 lane pick, 8 element pick, 9 end.  Entry 0: rounds of
-                          the search that needed block-wide sums (bits 0-15); the one-CTA-per-row kernel adds the outcome
-                          of its search on integer masses in bits 16-19 (1 settled, 2 list too short, 0 undecided or not tried) */
+                          the search that needed block-wide sums (bits 0-15); bits 16-19: outcome of the search on integer
+                          masses (1 settled, 2 list too short, 0 undecided or not tried); bit 20, one-CTA-per-row kernel:
+                          the list was short enough for it */
 } rs_trace;
 
 /*

@@ -1179,7 +1179,7 @@ __global__ void __launch_bounds__(kLanes / LPT, (LPT >= 4 ? 2 : 1)) rowcta_kerne
         tr.ncand = ncand;
 #pragma unroll
         for (int i = 0; i < 10; i++) tr.t_ns[i] = ts[i];
-        tr.t_ns[0] = n_eval | ((uint32_t)quick << 16) | (ncand <= (uint32_t)kQuickCap ? 0x100000u : 0u);
+        tr.t_ns[0] = n_eval | ((uint32_t)quick << 16) | (ncand <= kListCap ? 0x100000u : 0u);
         p.dbg_trace[b] = tr;
     }
 }

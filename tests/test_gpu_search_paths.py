@@ -56,18 +56,33 @@ def test_rows_of_which_nothing_is_cut_off(abi, mode, kind, B, V, temp):
         check_against_oracle(abi, make_logits(kind, B, V, 12, torch), 6, temp, -1, 1.0, mode, pen=pen)
 
 
-@pytest.mark.parametrize("mode", [2, 3, 4])
+@pytest.mark.parametrize("mode", [2, 3, 4, 5, 6])    # streaming, on-chip, one CTA per row; exact search only in the last two
 @pytest.mark.parametrize("kind,V,k,p", [("normal3", 4, -1, 0.5), ("uniform", 28, 5, 0.9), ("coarse", 64, -1, 0.6), ("equal", 508, 40, 0.3),
                                         ("uniform", 512, -1, 0.95), ("coarse", 512, 100, 1.0), ("uniform", 516, 200, 0.99),
                                         ("peaked", 50304, 1, 1.0), ("normal3", 100256, 50, 1e-7), ("coarse", 32768, 250, 0.9)])
 def test_integer_search_by_rank(abi, mode, kind, V, k, p):
-    """Candidate lists shorter than the sample, of exactly and just over the longest length, made of few distinct values,
-    all equal, cut by the count alone, and a top_p inside the margin of the empty set."""
+    """Candidate lists shorter than the sample, around the longest length, made of few distinct values, all equal, cut by the
+    count alone, and a top_p inside the margin of the empty set."""
     for seed in (1, 2):
         check_against_oracle(abi, make_logits(kind, 6, V, seed, torch), seed, 0.9, k, p, mode)
 
 
-@pytest.mark.parametrize("mode", [0, 1, 2, 3])        # the planner's choice, whole row only, streaming, on-chip
+@pytest.mark.parametrize("mode,rep,longest", [(2, False, 512), (3, True, 512), (4, True, 512), (4, False, 1024)])
+def test_longest_list_of_the_integer_search(abi, mode, rep, longest):
+    """Rows whose list is the whole row, of just under, exactly and just over the longest length: settled on integer masses
+    up to it, by the exact search beyond.  (One CTA per row without penalties holds twice the length.)"""
+    for V in (longest - 4, longest, longest + 4):
+        pen = torch.rand(6, V, generator=torch.Generator().manual_seed(4)) * 0.5 if rep else None
+        tr = check_against_oracle(abi, make_logits("uniform", 6, V, 71, torch), 3, 0.9, -1, 0.95, mode, pen=pen, rows=6)
+        for t in tr:
+            assert t.ncand == V and t.path == 0
+            outcome, rounds = (t.t_ns[0] >> 16) & 0xf, t.t_ns[0] & 0xffff
+            assert (outcome, rounds > 0) == ((1, False) if V <= longest else (0, True)), (V, outcome, rounds)
+            if mode == 4:
+                assert (t.t_ns[0] >> 20) & 1 == (1 if V <= longest else 0)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3, 5, 6])  # the planner's choice, whole row only, streaming, on-chip; exact search only
 @pytest.mark.parametrize("kind,B,V,temp,k,p", [("normal3", 2, 16384, 1.0, -1, 0.9), ("normal3", 3, 16388, 1.0, -1, 0.99),
                                                ("peaked", 130, 50304, 1.0, -1, 0.95), ("uniform", 2, 131072, 1.0, -1, 0.5),
                                                ("uniform", 4, 20484, 0.7, -1, 0.999999), ("normal3", 3, 65536, 0.8, 1000, 0.95),
