@@ -134,8 +134,7 @@ __device__ __forceinline__ void slab_pass(const Row<C, SMEM>& row, int& n, const
 // entries of the list as sample, each lane sums the sets of one of them (quick_sample: the list is split over the warps
 // of the CTA), which leaves about a thirty-second of the list between the highest sample that exceeds and the lowest
 // that passes; one warp ranks those against each other (quick_settle).  Bound by the latency of one warp: replaying the
-// loop with a scan of the list in each of its ~14 rounds took 2 us longer (a call of B=1, V=262144: 20.0 -> 18.2 us;
-// B=160, V=100256, bf16: 51.0 -> 46.7 us).
+// loop with a scan of the list in each of its ~14 rounds took 2 us longer (a call of B=1, V=262144: 20.0 -> 18.2 us).
 struct QuickTest {       // the three possible outcomes of the reference's tests at a set of count c and mass m
     bool use_cnt;
     uint32_t top_k, tp_lo, tp_hi, margin;
