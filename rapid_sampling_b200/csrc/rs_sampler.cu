@@ -1312,16 +1312,19 @@ __device__ __forceinline__ bool row_args_one(int b, int V, const float* temperat
     out[b] = r;
     return !(k >= V && pp >= 1.0f) && (sel == 0 || k >= V);
 }
-// route (calls of one block only): whether any row does
 __global__ void row_args_kernel(int B, int V, const float* temperature, const int* top_k, const float* top_p, int rep,
-                                int allow_candidates, RowArgs* out, int* status, int* status_mirror, int* route) {
+                                int allow_candidates, RowArgs* out, int* status, int* status_mirror) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < B) row_args_one(b, V, temperature, top_k, top_p, rep, allow_candidates, out, status, status_mirror);
+}
+// The same in one block, which also writes whether any row searches widely.
+__global__ void row_args_route_kernel(int B, int V, const float* temperature, const int* top_k, const float* top_p, int rep,
+                                      int allow_candidates, RowArgs* out, int* status, int* status_mirror, int* route) {
     int wide = 0;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x)
+    for (int b = threadIdx.x; b < B; b += blockDim.x)
         wide |= row_args_one(b, V, temperature, top_k, top_p, rep, allow_candidates, out, status, status_mirror) ? 1 : 0;
-    if (route) {
-        wide = __syncthreads_or(wide);
-        if (threadIdx.x == 0) *route = wide ? 1 : 0;
-    }
+    wide = __syncthreads_or(wide);
+    if (threadIdx.x == 0) *route = wide ? 1 : 0;
 }
 
 // ------------------------------------------------------------------ host side -------------
@@ -1650,8 +1653,13 @@ static int sample_rows_impl(const void* logits, int dtype, int64_t B, int64_t T,
     cudaStream_t st = (cudaStream_t)stream;
     RowArgs* rows = (RowArgs*)((char*)workspace + 256);
     int* route = either ? (int*)workspace + 16 : nullptr;      // (in the 256 bytes of the status word)
-    row_args_kernel<<<either ? 1u : (unsigned)((B + 127) / 128), either ? 1024 : 128, 0, st>>>(
-        (int)B, (int)V, temperature, top_k, top_p, penalties ? 1 : 0, allow_cand ? 1 : 0, rows, (int*)workspace, di->mirror, route);
+    const int is_rep = penalties ? 1 : 0, is_cand = allow_cand ? 1 : 0;
+    if (either)
+        row_args_route_kernel<<<1, 1024, 0, st>>>((int)B, (int)V, temperature, top_k, top_p, is_rep, is_cand, rows, (int*)workspace,
+                                                  di->mirror, route);
+    else
+        row_args_kernel<<<(unsigned)((B + 127) / 128), 128, 0, st>>>((int)B, (int)V, temperature, top_k, top_p, is_rep, is_cand, rows,
+                                                                     (int*)workspace, di->mirror);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "launch(row_args)");
     g_launches.fetch_add(1, std::memory_order_relaxed);
