@@ -652,7 +652,10 @@ __global__ void __launch_bounds__(kLanes / C, MORE_REGS ? 6 : ctas_per_sm_by_reg
     }
     // neither more than top_k elements nor (clear of the roundings) the mass: no cutoff lies above the bound
     if (!enough && cmass < a_top_p * 0.99999f) cand_ok = false;
-    if (want_hist && wl == 0) qsum[lane] = qsum[lane + 32] = 0u;
+    if (want_hist) {
+        __syncthreads();      // every warp's additions are done (an exchange counts arrived bytes, it orders nothing else)
+        if (wl == 0) qsum[lane] = qsum[lane + 32] = 0u;
+    }
     // division is monotone, so the row's min/max probability are the quotients of min/max e
     const float pmin = emin / denom, pmax = emax / denom;
     if (p.dbg_probs) {   // test instrumentation: the probabilities of the whole row

@@ -106,7 +106,7 @@ def test_both_search_strategies_are_exercised(abi):
 
 
 def test_row_cta_integer_search_and_its_hand_over_to_exact_sums(abi, ref):
-    """The one-CTA-per-row kernel first runs the search in one warp on exact integer masses and keeps the result only
+    """The one-CTA-per-row kernel first runs the search on exact integer masses and keeps the result only
     if no mass came within the fp32 rounding of the reference's sums of top_p.  Ordinary rows must be settled that
     way; with top_p set to the very mass of a prefix of the sorted row the integer search must stand back and the
     block-wide search on fp32 sums must give the reference's ids, trace for trace."""
